@@ -113,6 +113,12 @@ struct PcgState {
 constexpr uint32_t kLongBlockTerms = 1024;
 constexpr int kLongLanes = 32;
 
+// Problems of at most this many tile rows (128 cameras) are solved by the
+// cluster kernels of vlba_pcg_small.cu, the others by the persistent k_pcg; a
+// problem's kernel follows from its own size, the same alone and in any batch.
+constexpr uint32_t kSmallPcgRows = 16;
+constexpr int kSmallPcgClasses = 4;
+
 // Everything the kernels touch.  Passed by value.
 struct Dev {
   // sizes
@@ -133,7 +139,13 @@ struct Dev {
   const uint32_t* prob_pose_begin;   // [num_problems + 1]
   const uint32_t* prob_point_begin;  // [num_problems + 1]
   const uint32_t* prob_tr_begin;     // tile rows [num_problems + 1]
+  const uint32_t* prob_tile_begin;   // tiles [num_problems + 1]
   const uint32_t* prob_chunk_begin;  // point chunks [num_problems + 1]
+  // The problems of the small PCG kernels by class (small_pcg_class), and how
+  // many problems the persistent kernel solves.
+  const uint32_t* small_list;
+  uint32_t small_off[kSmallPcgClasses + 1];
+  uint32_t num_big;
   const uint32_t* pose_prob;         // [num_poses]
   const uint32_t* point_prob;        // [num_points]
   const uint32_t* slot_prob;         // [num_var_cams]

@@ -2282,7 +2282,13 @@ __global__ void __launch_bounds__(1024) k_pcg_setup(Dev d) {
   __syncthreads();
   unsigned int mine = 0;
   for (uint32_t P = threadIdx.x; P < d.num_problems; P += blockDim.x) {
-    const bool on = !d.ctrl[P].done && d.prob_tr_begin[P + 1] > d.prob_tr_begin[P];
+    // The small problems' states are their own kernels'.
+    const uint32_t rows = d.prob_tr_begin[P + 1] - d.prob_tr_begin[P];
+    if (rows <= kSmallPcgRows) {
+      d.pcg[P].active = 0u;
+      continue;
+    }
+    const bool on = !d.ctrl[P].done;
     PcgState& s = d.pcg[P];
     s.active = on ? 1u : 0u;
     s.iters = 0u;
@@ -2368,11 +2374,6 @@ cudaError_t launch_cam_diag(const Dev& d, cudaStream_t s) {
 
 cudaError_t launch_pose_update(const Dev& d, cudaStream_t s) {
   k_pose_update<<<grid1d(d.num_poses, 256), 256, 0, s>>>(d);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_pcg_setup(const Dev& d, cudaStream_t s) {
-  k_pcg_setup<<<1, 1024, 0, s>>>(d);
   return cudaGetLastError();
 }
 
@@ -2476,7 +2477,11 @@ int pcg_grid_size(int, int sm_count) {
 }
 
 cudaError_t launch_pcg(const Dev& d, int grid, cudaStream_t s) {
-  if (d.num_tile_rows == 0) return cudaSuccess;
+  cudaError_t e = launch_pcg_small(d, s);
+  if (e != cudaSuccess || d.num_big == 0) return e;
+  k_pcg_setup<<<1, 1024, 0, s>>>(d);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
   void* args[] = {const_cast<Dev*>(&d)};
   return cudaLaunchCooperativeKernel((const void*)k_pcg, grid, Pcg::kThreads, args, Pcg::kSmem, s);
 }

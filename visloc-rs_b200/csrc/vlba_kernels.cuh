@@ -23,9 +23,14 @@ cudaError_t launch_block_order(const Dev& d, cudaStream_t s);
 cudaError_t launch_pair_points(const Dev& d, uint64_t n, cudaStream_t s);
 // cam_pt[i] = obs_point[cam_obs[i]] for the n listed observations.
 cudaError_t launch_cam_points(const Dev& d, uint32_t n, cudaStream_t s);
-cudaError_t launch_pcg(const Dev& d, int sm_count, cudaStream_t s);
+// The PCG of every problem: the small ones' cluster kernels, then (when the
+// plan has larger ones) the persistent kernel on `grid` blocks.
+cudaError_t launch_pcg(const Dev& d, int grid, cudaStream_t s);
+// The small problems alone (vlba_pcg_small.cu).
+cudaError_t launch_pcg_small(const Dev& d, cudaStream_t s);
+// Class of a problem of `rows` tile rows, or -1 for the persistent kernel.
+int small_pcg_class(uint32_t rows);
 cudaError_t launch_pose_update(const Dev& d, cudaStream_t s);
-cudaError_t launch_pcg_setup(const Dev& d, cudaStream_t s);
 // Fill the tiles, preconditioner and rhs of a reduced system given directly
 // (device arrays in the reference's layout; the off-diagonal blocks f32, or
 // f64 when offdiag is null).

@@ -1,0 +1,317 @@
+// vlba_pcg_small.cu -- block-Jacobi PCG on the reduced systems of small
+// problems (at most kSmallPcgRows tile rows, 128 cameras), one thread-block
+// cluster per problem.
+//
+// The persistent k_pcg (vlba_kernels.cu) streams tiles of S and crosses two
+// grid barriers in each iteration: 5-6 us for a 20-keyframe window whatever
+// its size, nearly all of it waiting.  Here S lives in registers for the whole
+// solve and an iteration crosses two barriers of one cluster (of one block
+// for up to 16 cameras), the same recurrence and stopping rule:
+//
+//   one warp per camera: lane l holds columns l, l + 32, ... of the camera's
+//   six rows of S, and its own copy of those entries of p;
+//   q = S p      each lane's partial products, then a reduce-scatter butterfly
+//   -- barrier: every warp's p.q
+//   x, r, z of the camera on lanes 0-5; z pushed to every block of the
+//   cluster through distributed shared memory
+//   -- barrier: z, and every warp's r.z and r.r
+//   p = z + beta p, on every lane for its columns.
+//
+// What bounds it is the chain of one iteration (LDS, FMA, shuffles, barrier),
+// so the cluster is as small as the registers allow: 3 columns per lane up to
+// 16 cameras (one block), 6 up to 32 (two), 12 up to 64 (four blocks of 16
+// warps, 72 registers of S per thread) and 24 up to 128 (sixteen blocks of 8
+// warps, 144 registers).  Whole LM solves from host arrays on B200, k_pcg
+// against this kernel: a 20-keyframe window (10 LM iterations) 5.19 -> 2.90
+// ms, 50 cameras (20) 9.9 -> 5.3 ms, GNC on 60 cameras 31.7 -> 19.4 ms, 48
+// windows in one batch (6) 8.35 -> 6.27 ms.
+//
+// Every sum runs in an order fixed by the problem's own size, so a problem
+// solves the same alone and in any batch.  The cluster's blocks compute the
+// same scalars from the same slots and leave the loop together.
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "vlba_common.cuh"
+#include "vlba_kernels.cuh"
+
+namespace vlba {
+namespace {
+
+__device__ __forceinline__ double warp_sum_all(double v) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
+}
+// Sum over lanes 0-7 (lanes 6 and 7 hold zero), in lane 0 and its group.
+__device__ __forceinline__ double group_sum(double v) {
+#pragma unroll
+  for (int off = 4; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
+}
+
+// Address of `p` (in this block's shared memory) in block `rank` of the cluster.
+__device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+               : "=r"(a)
+               : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void st_peer(uint32_t a, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void st_peer(uint32_t a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
+// Barrier over the problem's blocks: the stores before it (also those into
+// other blocks' shared memory) are visible after it.
+template <int C>
+__device__ __forceinline__ void team_barrier() {
+  if (C == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
+
+// C blocks of W warps, one camera per warp; CPL columns of S per lane
+// (32 CPL = 6 C W).
+template <int C, int W, int CPL>
+__global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* list) {
+  constexpr int kNodes = C * W, kRows = kNodes / 8;
+  static_assert(32 * CPL == 6 * kNodes, "a lane's columns cover the system");
+  __shared__ float zs[32 * CPL];
+  __shared__ double s_pq[kNodes], s_rz[kNodes], s_rr[kNodes];
+  __shared__ uint32_t tmap[kRows * kRows];  // tile of (I, J), J <= I
+  const uint32_t P = list[blockIdx.x / C];
+  if (d.ctrl[P].done) return;  // the same for every block of the cluster
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t rank = C == 1 ? 0u : blockIdx.x % C;
+  const uint32_t node = rank * W + warp;
+  const uint32_t tr0 = d.prob_tr_begin[P], rows = d.prob_tr_begin[P + 1] - tr0;
+  const uint32_t nodes = rows * 8u;  // padded slots have zero rows and rhs
+  const bool mine = node < nodes;
+
+  for (uint32_t i = threadIdx.x; i < (uint32_t)(kRows * kRows); i += 32 * W) tmap[i] = kNone;
+  __syncthreads();
+  for (uint32_t t = d.prob_tile_begin[P] + threadIdx.x; t < d.prob_tile_begin[P + 1]; t += 32 * W) {
+    const uint32_t ij = d.tile_ij[t];
+    tmap[((ij >> 16) - tr0) * kRows + ((ij & 0xFFFFu) - tr0)] = t;
+  }
+  __syncthreads();
+
+  // The camera's six rows of S: from the tile right of (or on) the diagonal
+  // of its tile row, else the mirrored block of the lower tile.
+  float S[6][CPL], p[CPL];
+#pragma unroll
+  for (int j = 0; j < CPL; ++j) {
+    const uint32_t col = lane + 32u * j, cn = col / 6u, c = col % 6u;
+    p[j] = 0.0f;
+#pragma unroll
+    for (int r = 0; r < 6; ++r) S[r][j] = 0.0f;
+    if (mine && cn < nodes) {
+      const uint32_t I = node >> 3, J = cn >> 3;
+      const bool lower = I >= J;
+      const uint32_t t = lower ? tmap[I * kRows + J] : tmap[J * kRows + I];
+      if (t != kNone) {
+        const float* tile = d.tiles + (size_t)t * (64 * kBlock);
+        if (lower) {
+          const float* b = tile + ((node & 7u) * 8u + (cn & 7u)) * kBlock + c;
+#pragma unroll
+          for (int r = 0; r < 6; ++r) S[r][j] = b[6 * r];
+        } else {
+          const float2* b =
+              reinterpret_cast<const float2*>(tile + ((cn & 7u) * 8u + (node & 7u)) * kBlock + c * 6u);
+#pragma unroll
+          for (int r = 0; r < 3; ++r) {
+            const float2 v = b[r];
+            S[2 * r][j] = v.x;
+            S[2 * r + 1][j] = v.y;
+          }
+        }
+      }
+    }
+  }
+
+  // The camera's vector entries on lanes 0-5 (zero on the others).
+  const uint32_t a = lane < 6u ? lane : 0u;
+  const bool own = mine && lane < 6u;
+  const size_t at = (size_t)6 * (8u * tr0 + node) + a;
+  float m[6];
+#pragma unroll
+  for (int b = 0; b < 6; ++b) m[b] = own ? d.minv[6 * at + b] : 0.0f;
+  float x = 0.0f, r = own ? d.rhs[at] : 0.0f, z, po = 0.0f;
+  auto precondition = [&]() {
+    z = 0.0f;
+#pragma unroll
+    for (int b = 0; b < 6; ++b) z += m[b] * __shfl_sync(0xffffffffu, r, b);
+  };
+  // z and the camera's r.z and r.r into every block of the cluster.
+  auto publish = [&]() {
+    const double rz = group_sum((double)r * (double)z), rr = group_sum((double)r * (double)r);
+    if (C == 1) {
+      if (lane < 6u) zs[6 * node + lane] = z;
+      if (lane == 0) {
+        s_rz[node] = rz;
+        s_rr[node] = rr;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 6 * C; i += 32) {
+        const uint32_t e = lane + i, peer = e / 6u, q = e % 6u;
+        const float v = __shfl_sync(0xffffffffu, z, q);
+        if (e < 6u * C) st_peer(peer_addr(&zs[6 * node + q], peer), v);
+      }
+      const double rz0 = __shfl_sync(0xffffffffu, rz, 0), rr0 = __shfl_sync(0xffffffffu, rr, 0);
+      if (lane < (uint32_t)C) {
+        st_peer(peer_addr(&s_rz[node], lane), rz0);
+        st_peer(peer_addr(&s_rr[node], lane), rr0);
+      }
+    }
+  };
+  auto sum = [&](const double* s) {
+    double v = 0.0;
+#pragma unroll
+    for (int i = 0; i < kNodes; i += 32)
+      if (lane + i < (uint32_t)kNodes) v += s[lane + i];
+    return warp_sum_all(v);
+  };
+
+  precondition();
+  if (C > 1) team_barrier<C>();  // every block runs before its memory is written
+  publish();
+  team_barrier<C>();
+  double rz = sum(s_rz), rr = sum(s_rr);
+  const LmParams& lp = d.params[P];
+  const double bnorm = sqrt(rr);
+  const double stop = lp.pcg_relative_tolerance * bnorm;
+  const uint32_t cap = lp.max_pcg_iterations;
+  uint32_t iters = 0, status = 0;
+  // pcg_init (ba.wgsl:420-439): done when |b| = 0 or r.z <= 0.
+  if (rr > 0.0 && rz > 0.0 && cap != 0u) {
+    float beta = 0.0f;
+    for (;;) {
+      float acc[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int j = 0; j < CPL; ++j) {
+        p[j] = __fmaf_rn(beta, p[j], zs[lane + 32 * j]);
+#pragma unroll
+        for (int q = 0; q < 6; ++q) acc[q] = __fmaf_rn(S[q][j], p[j], acc[q]);
+      }
+      po = __fmaf_rn(beta, po, z);
+      // Row sums over the lanes: a reduce-scatter (bit 4 keeps three of the
+      // six rows, bit 3 two or one of those), then a butterfly; then row a
+      // back to lane a.
+      const bool b4 = (lane >> 4) & 1u, b3 = (lane >> 3) & 1u;
+      float h[3];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const float keep = b4 ? acc[q + 3] : acc[q], send = b4 ? acc[q] : acc[q + 3];
+        h[q] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+      }
+      const float g0 = __shfl_xor_sync(0xffffffffu, b3 ? h[0] : h[2], 8);
+      const float g1 = __shfl_xor_sync(0xffffffffu, h[1], 8);
+      float u = b3 ? h[2] + g0 : h[0] + g0, v = h[1] + g1;  // v: rows 1 and 4, where b3 is 0
+#pragma unroll
+      for (int off = 4; off > 0; off >>= 1) {
+        u += __shfl_xor_sync(0xffffffffu, u, off);
+        v += __shfl_xor_sync(0xffffffffu, v, off);
+      }
+      const uint32_t part = a >= 3u ? a - 3u : a;
+      const uint32_t src = (a >= 3u ? 16u : 0u) + (part == 2u ? 8u : 0u);
+      const float qu = __shfl_sync(0xffffffffu, u, src), qv = __shfl_sync(0xffffffffu, v, src);
+      const float qa = own ? (part == 1u ? qv : qu) : 0.0f;
+      const double pq_node = group_sum((double)po * (double)qa);
+      if (C == 1) {
+        if (lane == 0) s_pq[node] = pq_node;
+      } else {
+        const double v0 = __shfl_sync(0xffffffffu, pq_node, 0);
+        if (lane < (uint32_t)C) st_peer(peer_addr(&s_pq[node], lane), v0);
+      }
+      team_barrier<C>();
+      const double pq = sum(s_pq);
+      if (!(pq > 0.0) || !isfinite(pq)) {
+        status = 2;  // non-positive curvature: x unchanged
+        break;
+      }
+      const float alpha = (float)(rz / pq);
+      x = x + alpha * po;
+      r = r - alpha * qa;
+      precondition();
+      publish();
+      team_barrier<C>();
+      const double rz_new = sum(s_rz);
+      rr = sum(s_rr);
+      ++iters;
+      if (sqrt(rr) <= stop || !(rz_new > 0.0)) {
+        rz = rz_new;
+        break;
+      }
+      if (iters >= cap) {
+        status = 1;
+        rz = rz_new;
+        break;
+      }
+      beta = (float)(rz_new / rz);
+      rz = rz_new;
+    }
+  }
+  if (own) d.x[at] = x;
+  if (rank == 0 && threadIdx.x == 0) {
+    PcgState& st = d.pcg[P];
+    st.iters = iters;
+    st.status = status;
+    st.bnorm = bnorm;
+    st.rnorm = sqrt(rr);
+    st.rz = rz;
+    st.active = 0u;
+  }
+}
+
+template <int C, int W, int CPL>
+cudaError_t launch_class(const Dev& d, uint32_t begin, uint32_t end, cudaStream_t s) {
+  if (begin == end) return cudaSuccess;
+  auto kernel = k_pcg_small<C, W, CPL>;
+  if (C > 8) {  // beyond the portable cluster size
+    const cudaError_t e =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(C * (end - begin));
+  cfg.blockDim = dim3(32 * W);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = C;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = C > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, d, d.small_list + begin);
+}
+
+}  // namespace
+
+int small_pcg_class(uint32_t rows) {
+  if (rows <= 2) return 0;
+  if (rows <= 4) return 1;
+  if (rows <= 8) return 2;
+  if (rows <= kSmallPcgRows) return 3;
+  return -1;
+}
+
+cudaError_t launch_pcg_small(const Dev& d, cudaStream_t s) {
+  cudaError_t e = launch_class<1, 16, 3>(d, d.small_off[0], d.small_off[1], s);
+  if (e == cudaSuccess) e = launch_class<2, 16, 6>(d, d.small_off[1], d.small_off[2], s);
+  if (e == cudaSuccess) e = launch_class<4, 16, 12>(d, d.small_off[2], d.small_off[3], s);
+  if (e == cudaSuccess) e = launch_class<16, 8, 24>(d, d.small_off[3], d.small_off[4], s);
+  return e;
+}
+
+}  // namespace vlba

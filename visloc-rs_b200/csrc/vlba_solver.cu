@@ -490,6 +490,19 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
   d.prob_point_begin = st.up(A, P.prob_point_begin);
   d.prob_tr_begin = st.up(A, P.prob_tr_begin);
   d.prob_chunk_begin = st.up(A, P.prob_chunk_begin);
+  // Each problem's tiles (contiguous, in problem order), and the problems of
+  // each small PCG class.
+  std::vector<uint32_t> tile_begin(P.num_problems + 1, 0u), small;
+  for (size_t t = 0; t < P.tile_ij.size(); ++t) ++tile_begin[P.tile_meta[4 * t + 3] + 1];
+  for (uint32_t p = 0; p < P.num_problems; ++p) tile_begin[p + 1] += tile_begin[p];
+  for (int k = 0; k < kSmallPcgClasses; ++k) {
+    for (uint32_t p = 0; p < P.num_problems; ++p)
+      if (small_pcg_class(P.prob_tr_begin[p + 1] - P.prob_tr_begin[p]) == k) small.push_back(p);
+    d.small_off[k + 1] = (uint32_t)small.size();
+  }
+  d.num_big = P.num_problems - (uint32_t)small.size();
+  d.prob_tile_begin = st.up(A, tile_begin);
+  d.small_list = st.up(A, small);
   d.pose_prob = st.up(A, P.pose_prob);
   d.point_prob = st.up(A, P.point_prob);
   d.slot_prob = st.up(A, P.slot_prob);
@@ -760,6 +773,16 @@ void dump_trace(Context* c) {
                  acc[4] / iters / 1e3, acc[5] / iters / 1e3, wall / iters / 1e3);
 }
 
+// Kernels of one LM iteration: linearize, point prep, pose update, cost and
+// decide always; off-diagonal (short and long blocks), camera-diagonal and
+// the PCG kernels when the system has them.
+uint64_t iteration_launches(const Dev& d) {
+  uint64_t n = 5 + (d.num_offdiag_blocks ? 1 : 0) + (d.num_long_blocks ? 1 : 0) +
+               (d.num_var_cams ? 1 : 0) + (d.num_big ? 2 : 0);
+  for (int k = 0; k < kSmallPcgClasses; ++k) n += d.small_off[k + 1] > d.small_off[k] ? 1 : 0;
+  return n;
+}
+
 // The device LM loop over all uploaded problems.
 // The kernels of one LM iteration (trial), in order; `ev` (4 events or null)
 // brackets the phases for profiling.  Returns the number of launches.
@@ -777,9 +800,8 @@ uint64_t enqueue_iteration(Context* c, cudaEvent_t* ev) {
   VLBA_CUDA(cudaEventRecord(c->join, c->side));
   check_launch(launch_offdiag(d, s), "off-diagonal blocks");
   VLBA_CUDA(cudaStreamWaitEvent(s, c->join, 0));
-  check_launch(launch_pcg_setup(d, s), "pcg setup");
   if (ev) VLBA_CUDA(cudaEventRecord(ev[2], s));
-  if (c->gate && d.num_tile_rows) {
+  if (c->gate && d.num_big) {
     std::lock_guard<std::mutex> lock(c->gate->mu);
     VLBA_CUDA(cudaStreamWaitEvent(s, c->gate->last, 0));
     check_launch(launch_pcg(d, c->pcg_grid, s), "pcg");
@@ -793,11 +815,7 @@ uint64_t enqueue_iteration(Context* c, cudaEvent_t* ev) {
   check_launch(launch_cost(d, true, s), "trial cost");
   check_launch(launch_decide(d, false, s), "decide");
   if (ev) VLBA_CUDA(cudaEventRecord(ev[4], s));
-  // linearize, point prep, pcg setup, pose update, cost, decide always;
-  // off-diagonal (short and long blocks), camera-diagonal and PCG kernels
-  // when the system has them.
-  return 6 + (d.num_offdiag_blocks ? 1 : 0) + (d.num_long_blocks ? 1 : 0) + (d.num_var_cams ? 1 : 0) +
-         (d.num_tile_rows ? 1 : 0);
+  return iteration_launches(d);
 }
 
 uint64_t enqueue_initial(Context* c) {
@@ -850,9 +868,7 @@ RunStats run_lm_graph(Context* c, uint32_t max_iters) {
   } else {
     launches = 3;
     for (uint32_t it = 0; it < max_iters; ++it) {
-      const Dev& d = c->dev;
-      launches += 6 + (d.num_offdiag_blocks ? 1 : 0) + (d.num_var_cams ? 1 : 0) +
-                  (d.num_tile_rows ? 1 : 0);
+      launches += iteration_launches(c->dev);
     }
   }
   VLBA_CUDA(cudaEventRecord(c->ev[0], s));
@@ -943,6 +959,7 @@ LaunchShape autotune(Context* c) {
   const int gmax = pcg_grid_max(c), gmin = std::max(1, pcg_grid_min(c));
   std::vector<int> grids;
   for (double f : {1.0, 0.75, 0.5, 0.375, 0.25, 0.125}) {
+    if (!d.num_big && !grids.empty()) break;  // the shape is the persistent kernel's
     const int g = std::max(gmin, (int)(f * gmax));
     if (std::find(grids.begin(), grids.end(), g) == grids.end()) grids.push_back(g);
   }
@@ -956,7 +973,6 @@ LaunchShape autotune(Context* c) {
       float ms = 1e30f;
       for (int rep = 0; rep < 3; ++rep) {
         VLBA_CUDA(cudaEventRecord(c->ev[0], s));
-        check_launch(launch_pcg_setup(d, s), "pcg setup");
         check_launch(launch_pcg(d, c->pcg_grid, s), "pcg");
         VLBA_CUDA(cudaEventRecord(c->ev[1], s));
         VLBA_CUDA(cudaEventSynchronize(c->ev[1]));
@@ -1800,7 +1816,6 @@ int visloc_ba_cuda_linear_step(void* ctx, const vlba_problem* problem, const vlb
     vlba::prepare_system(c, problem, config, lambda);
     vlba::Dev& d = c->dev;
     cudaStream_t s = c->stream;
-    vlba::check_launch(vlba::launch_pcg_setup(d, s), "pcg setup");
     vlba::check_launch(vlba::launch_pcg(d, c->pcg_grid, s), "pcg");
     if (d.trace) vlba::dump_trace(c);
     vlba::check_launch(vlba::launch_pose_update(d, s), "pose update");
@@ -2695,7 +2710,6 @@ int visloc_ba_cuda_reduced_solve(void* ctx, const vlba_reduced_system* sys, doub
     cudaStream_t s = c->stream;
     vlba::Dev& d = c->dev;
     VLBA_CUDA(cudaEventRecord(c->ev[2], s));
-    vlba::check_launch(vlba::launch_pcg_setup(d, s), "pcg setup");
     vlba::check_launch(vlba::launch_pcg(d, c->pcg_grid, s), "pcg");
     vlba::record_pcg_ms(c);
     vlba::PcgState pg;
