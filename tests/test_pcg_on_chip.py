@@ -1,0 +1,152 @@
+"""The PCG kernels of reduced systems that stay on the chip at the sizes where
+one begins and ends, against the FP64 iteration they restate: the clusters
+(at most 16 tile rows, 128 cameras), the teams of blocks (up to about 450
+densely coupled cameras), and past them the persistent kernel."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from visloc_ba import BaConfig, RobustKernel, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def system(n, keep, seed):
+    """A random SPD block system of n nodes, each pair coupled with
+    probability `keep`, its condition number about 50."""
+    rng = np.random.default_rng(seed)
+    a, b = np.triu_indices(n, 1)
+    on = rng.random(len(a)) <= keep
+    a, b = a[on], b[on]
+    ga, gb = (np.eye(6) + 0.3 * rng.standard_normal((len(a), 6, 6)) for _ in range(2))
+    off = -(gb.transpose(0, 2, 1) @ ga)
+    edges = np.stack([a, b], 1)
+    diag = np.zeros((n, 6, 6))
+    np.add.at(diag, a, ga.transpose(0, 2, 1) @ ga)
+    np.add.at(diag, b, gb.transpose(0, 2, 1) @ gb)
+    diag += np.eye(6) * (1.0 + 0.05 * np.trace(diag.mean(0)) / 6)
+    return diag, edges.astype(np.uint32), off.astype(np.float32), rng.standard_normal((n, 6))
+
+
+def dense(diag, edges, off):
+    n = len(diag)
+    S = np.zeros((n, 6, n, 6))
+    S[np.arange(n), :, np.arange(n), :] = diag
+    a, b = edges[:, 0], edges[:, 1]
+    S[b, :, a, :] = off
+    S[a, :, b, :] = off.transpose(0, 2, 1)
+    return S.reshape(6 * n, 6 * n)
+
+
+def pcg64(S, diag, rhs, tol, cap):
+    n = len(diag)
+    inv = np.linalg.inv(diag)
+    prec = lambda r: np.einsum("nab,nb->na", inv, r.reshape(n, 6)).reshape(-1)  # noqa: E731
+    b = rhs.reshape(-1)
+    x, r = np.zeros_like(b), b.copy()
+    z = prec(r)
+    p, rz = z.copy(), r @ z
+    for k in range(cap):
+        q = S @ p
+        alpha = rz / (p @ q)
+        x += alpha * p
+        r -= alpha * q
+        if np.linalg.norm(r) <= tol * np.linalg.norm(b):
+            return x, k + 1
+        z = prec(r)
+        new = r @ z
+        p, rz = z + (new / rz) * p, new
+    return x, cap
+
+
+@pytest.mark.parametrize("n", [1, 2, 5, 8, 15, 16, 17, 31, 32, 33, 63, 64, 65, 71, 127, 128, 129, 151, 256,
+                               330, 449, 490])
+@pytest.mark.parametrize("keep", [1.0, 0.15])
+def test_matches_the_fp64_iteration(solver, n, keep):
+    diag, edges, off, rhs = system(n, keep, 7 * n)
+    S = dense(diag, edges, off)
+    x, it, rr = solver.reduced_solve(diag, edges, off, rhs, 1e-5, 300)
+    ref, it_ref = pcg64(S, diag, rhs, 1e-5, 300)
+    assert abs(it - it_ref) <= 1 and rr <= 1e-5
+    # Both stop within 1e-5 |b| of the solution's residual: they differ by
+    # at most twice that over the smallest eigenvalue, and FP32 rounding.
+    lmin = np.linalg.eigvalsh(S)[0]
+    bound = 2e-5 * np.linalg.norm(rhs) / lmin + 1e-5 * np.linalg.norm(ref)
+    assert np.linalg.norm(x.reshape(-1) - ref) <= bound
+    # A few iterations only: the iterates themselves, before rounding grows.
+    if n >= 5:
+        x3, it3, _ = solver.reduced_solve(diag, edges, off, rhs, 0.0, 3)
+        ref3, _ = pcg64(S, diag, rhs, -1.0, 3)
+        assert it3 == 3
+        assert np.linalg.norm(x3.reshape(-1) - ref3) <= 1e-5 * np.linalg.norm(ref3)
+    # The same bits on a repeated call.
+    again, _, _ = solver.reduced_solve(diag, edges, off, rhs, 1e-5, 300)
+    assert np.array_equal(again, x)
+
+
+@pytest.mark.parametrize("n", [3, 20, 50, 100, 140, 480])
+def test_stopping_rules(solver, n):
+    """Zero right-hand side, iteration cap 0 and 1, non-positive curvature
+    (x stays at the last iterate) and NaN: as the persistent kernel."""
+    diag, edges, off, rhs = system(n, 0.5, n)
+    x, it, _ = solver.reduced_solve(diag, edges, off, 0.0 * rhs, 1e-6, 50)
+    assert it == 0 and not x.any()
+    x, it, _ = solver.reduced_solve(diag, edges, off, rhs, 1e-6, 0)
+    assert it == 0 and not x.any()
+    x, it, _ = solver.reduced_solve(diag, edges, off, rhs, 1e-12, 1)
+    assert it == 1 and x.any()
+    # Indefinite beyond the block diagonal: large couplings.
+    x, it, _ = solver.reduced_solve(diag, edges, 100.0 * off, rhs, 1e-6, 50)
+    assert it < 50 and np.isfinite(x).all()
+    bad = rhs.copy()
+    bad[0, 0] = np.nan
+    x, it, _ = solver.reduced_solve(diag, edges, off, bad, 1e-6, 50)
+    assert it == 0 and not x.any()
+
+
+@pytest.mark.parametrize("band", [2, 9, 40])
+def test_banded_team(solver, band):
+    """A long chain (1,400 nodes, more tile rows than blocks at the widest
+    team): each block reads its own stretch of columns."""
+    n = 1400
+    rng = np.random.default_rng(band)
+    a = np.repeat(np.arange(n), band)
+    b = a + np.tile(np.arange(1, band + 1), n)
+    edges = np.stack([a, b], 1)[b < n]
+    a, b = edges[:, 0], edges[:, 1]
+    ga, gb = (np.eye(6) + 0.3 * rng.standard_normal((len(a), 6, 6)) for _ in range(2))
+    off = -(gb.transpose(0, 2, 1) @ ga).astype(np.float32)
+    diag = np.tile(np.eye(6) * 0.5, (n, 1, 1))
+    np.add.at(diag, a, ga.transpose(0, 2, 1) @ ga)
+    np.add.at(diag, b, gb.transpose(0, 2, 1) @ gb)
+    rhs = rng.standard_normal((n, 6))
+    x, it, _ = solver.reduced_solve(diag, edges, off, rhs, 0.0, 4)
+    ref, _ = pcg64(dense(diag, edges, off), diag, rhs, -1.0, 4)
+    assert it == 4
+    assert np.linalg.norm(x.reshape(-1) - ref) <= 1e-5 * np.linalg.norm(ref)
+
+
+def test_teams_solve_the_same_alone_and_in_a_batch(solver):
+    """Problems of every PCG kernel in one batch (teams in two rounds): the
+    bits of each solved alone."""
+    probs = [synth.ring_problem(140, 6000, seed=1), synth.stereo_window(20, 800, seed=2),
+             synth.ring_problem(200, 8000, seed=3), synth.ring_problem(300, 20000, seed=4),
+             synth.street_loop(500, 20000, seed=5), synth.ring_problem(100, 4000, seed=6)]
+    cfg = BaConfig(max_iterations=4, robust_kernel=RobustKernel.huber(1.0), max_pcg_iterations=60,
+                   pcg_relative_tolerance=1e-6)
+    alone = [p.copy() for p in probs]
+    costs = []
+    for p in alone:
+        st, res = solver.optimize(p, cfg)
+        assert st == 0
+        costs.append(res.final_cost)
+    for graph in (False, True):
+        cfg.graph = graph
+        batch = [p.copy() for p in probs]
+        statuses, results = solver.batch_optimize(batch, cfg)
+        assert statuses == [0] * len(probs)
+        for a, b, c, r in zip(alone, batch, costs, results):
+            assert r.final_cost == c
+            assert np.array_equal(a.pose_q, b.pose_q) and np.array_equal(a.landmarks, b.landmarks)

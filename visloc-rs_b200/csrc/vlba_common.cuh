@@ -119,6 +119,21 @@ constexpr int kLongLanes = 32;
 constexpr uint32_t kSmallPcgRows = 16;
 constexpr int kSmallPcgClasses = 4;
 
+constexpr uint32_t kLineWords = 16;  // 64-bit words of a 128-byte line
+
+// One block of a problem's team (vlba_pcg_team.cu).
+struct TeamCta {
+  uint32_t prob;
+  uint32_t rank, size;    // block of the team, blocks in it
+  uint32_t node0, node1;  // its cameras (slots of the problem)
+  uint32_t ncols;         // tile columns its rows read
+  uint32_t col_begin;     // into team_cols: those columns, ascending
+  uint32_t ent_begin;     // into team_ents: the tile of (tile row, column), or kNone
+  uint32_t slot_base;     // the team's first exchange slot, and block of team_cta
+  uint32_t z_own;         // its z words, after the team's
+  uint64_t z_team;        // the team's first z word
+};
+
 // Everything the kernels touch.  Passed by value.
 struct Dev {
   // sizes
@@ -146,6 +161,17 @@ struct Dev {
   const uint32_t* small_list;
   uint32_t small_off[kSmallPcgClasses + 1];
   uint32_t num_big;
+  // The problems solved by teams of blocks: team_rounds rounds of team_grid
+  // blocks, each entry of team_sched a block of team_cta or kNone.
+  uint32_t team_rounds, team_grid, team_smem, team_slots_total;
+  const TeamCta* team_cta;
+  const uint32_t* team_sched;
+  const uint32_t* team_cols;
+  const uint32_t* team_ents;
+  unsigned long long* team_z;      // (exchange number, z), each block's on lines of its own
+  unsigned long long* team_slots;  // [2 kLineWords team_slots_total] (number, half of a double)
+  uint32_t* team_epoch;            // [num_problems] last exchange number used
+  const uint8_t* prob_big;         // [num_problems] 1: the persistent kernel's
   const uint32_t* pose_prob;         // [num_poses]
   const uint32_t* point_prob;        // [num_points]
   const uint32_t* slot_prob;         // [num_var_cams]
@@ -273,6 +299,16 @@ __device__ __forceinline__ unsigned long long now_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
+}
+
+// 1 / v for a positive normal v, to about two units in the last place: the
+// hardware's approximation and two Newton steps, a third of the latency of
+// the divide (the PCG's scalar chain).
+__device__ __forceinline__ double inverse64(double v) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+  y = fma(y, fma(-v, y, 1.0), y);
+  return fma(y, fma(-v, y, 1.0), y);
 }
 #endif
 

@@ -2282,9 +2282,8 @@ __global__ void __launch_bounds__(1024) k_pcg_setup(Dev d) {
   __syncthreads();
   unsigned int mine = 0;
   for (uint32_t P = threadIdx.x; P < d.num_problems; P += blockDim.x) {
-    // The small problems' states are their own kernels'.
-    const uint32_t rows = d.prob_tr_begin[P + 1] - d.prob_tr_begin[P];
-    if (rows <= kSmallPcgRows) {
+    // The other problems' states are their own kernels'.
+    if (!d.prob_big[P]) {
       d.pcg[P].active = 0u;
       continue;
     }
@@ -2478,6 +2477,7 @@ int pcg_grid_size(int, int sm_count) {
 
 cudaError_t launch_pcg(const Dev& d, int grid, cudaStream_t s) {
   cudaError_t e = launch_pcg_small(d, s);
+  if (e == cudaSuccess) e = launch_pcg_team(d, s);
   if (e != cudaSuccess || d.num_big == 0) return e;
   k_pcg_setup<<<1, 1024, 0, s>>>(d);
   e = cudaGetLastError();

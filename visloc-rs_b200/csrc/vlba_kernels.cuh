@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "vlba_common.cuh"
 
 namespace vlba {
@@ -23,13 +25,28 @@ cudaError_t launch_block_order(const Dev& d, cudaStream_t s);
 cudaError_t launch_pair_points(const Dev& d, uint64_t n, cudaStream_t s);
 // cam_pt[i] = obs_point[cam_obs[i]] for the n listed observations.
 cudaError_t launch_cam_points(const Dev& d, uint32_t n, cudaStream_t s);
-// The PCG of every problem: the small ones' cluster kernels, then (when the
-// plan has larger ones) the persistent kernel on `grid` blocks.
+// The PCG of every problem: the small ones' cluster kernels, the team kernel,
+// then (when the plan has larger ones) the persistent kernel on `grid` blocks.
 cudaError_t launch_pcg(const Dev& d, int grid, cudaStream_t s);
 // The small problems alone (vlba_pcg_small.cu).
 cudaError_t launch_pcg_small(const Dev& d, cudaStream_t s);
-// Class of a problem of `rows` tile rows, or -1 for the persistent kernel.
+// Class of a problem of `rows` tile rows, or -1 for a larger one.
 int small_pcg_class(uint32_t rows);
+
+// The problems past the small classes whose S fits the shared memory of a team
+// of blocks (vlba_pcg_team.cu): the teams' blocks and their rounds.
+struct TeamPlan {
+  std::vector<TeamCta> cta;
+  std::vector<uint32_t> sched, cols, ents;
+  std::vector<uint8_t> in_team;  // [num_problems]
+  uint32_t rounds = 0, grid = 0;
+  size_t smem = 0;  // the largest block's dynamic shared memory
+  uint64_t z_words = 0;
+};
+TeamPlan build_team_plan(const uint32_t* prob_tr_begin, uint32_t num_problems,
+                         const std::vector<uint32_t>& tile_ij,
+                         const std::vector<uint32_t>& tile_begin, uint32_t max_blocks);
+cudaError_t launch_pcg_team(const Dev& d, cudaStream_t s);
 cudaError_t launch_pose_update(const Dev& d, cudaStream_t s);
 // Fill the tiles, preconditioner and rhs of a reduced system given directly
 // (device arrays in the reference's layout; the off-diagonal blocks f32, or

@@ -55,9 +55,9 @@ __device__ __forceinline__ double group_sum(double v) {
 // Address of `p` (in this block's shared memory) in block `rank` of the cluster.
 __device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {
   uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-               : "=r"(a)
-               : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  asm("mapa.shared::cluster.u32 %0, %1, %2;"
+      : "=r"(a)
+      : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
   return a;
 }
 __device__ __forceinline__ void st_peer(uint32_t a, float v) {
@@ -84,9 +84,14 @@ __device__ __forceinline__ void team_barrier() {
 template <int C, int W, int CPL>
 __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* list) {
   constexpr int kNodes = C * W, kRows = kNodes / 8;
+  // Dot slots of a camera: its six products (a warp then sums them all, three
+  // butterfly levels fewer in the chain), or one sum where six would be more
+  // to push to every block than that saves (four blocks: 91 us a solve of 40
+  // cameras with sums, 106 with products).
+  constexpr int kPer = C <= 2 ? 6 : 1, kDots = kPer * kNodes;
   static_assert(32 * CPL == 6 * kNodes, "a lane's columns cover the system");
   __shared__ float zs[32 * CPL];
-  __shared__ double s_pq[kNodes], s_rz[kNodes], s_rr[kNodes];
+  __shared__ double s_pq[kDots], s_rz[kDots], s_rr[kDots];
   __shared__ uint32_t tmap[kRows * kRows];  // tile of (I, J), J <= I
   const uint32_t P = list[blockIdx.x / C];
   if (d.ctrl[P].done) return;  // the same for every block of the cluster
@@ -151,15 +156,24 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
 #pragma unroll
     for (int b = 0; b < 6; ++b) z += m[b] * __shfl_sync(0xffffffffu, r, b);
   };
-  // z and the camera's r.z and r.r into every block of the cluster.
+  // The camera's products v (lanes 0-5) into its slots of every block.
+  auto push = [&](double* slots, double v) {
+    if (kPer == 1) v = group_sum(v);
+    if (C == 1) {
+      if (lane < (uint32_t)kPer) slots[kPer * node + lane] = v;
+    } else {
+#pragma unroll
+      for (int i = 0; i < kPer * C; i += 32) {
+        const uint32_t e = lane + i, peer = e / (uint32_t)kPer, q = e % (uint32_t)kPer;
+        const double w = __shfl_sync(0xffffffffu, v, q);
+        if (e < (uint32_t)(kPer * C)) st_peer(peer_addr(&slots[kPer * node + q], peer), w);
+      }
+    }
+  };
+  // z and the products of r.z and r.r into every block of the cluster.
   auto publish = [&]() {
-    const double rz = group_sum((double)r * (double)z), rr = group_sum((double)r * (double)r);
     if (C == 1) {
       if (lane < 6u) zs[6 * node + lane] = z;
-      if (lane == 0) {
-        s_rz[node] = rz;
-        s_rr[node] = rr;
-      }
     } else {
 #pragma unroll
       for (int i = 0; i < 6 * C; i += 32) {
@@ -167,19 +181,21 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
         const float v = __shfl_sync(0xffffffffu, z, q);
         if (e < 6u * C) st_peer(peer_addr(&zs[6 * node + q], peer), v);
       }
-      const double rz0 = __shfl_sync(0xffffffffu, rz, 0), rr0 = __shfl_sync(0xffffffffu, rr, 0);
-      if (lane < (uint32_t)C) {
-        st_peer(peer_addr(&s_rz[node], lane), rz0);
-        st_peer(peer_addr(&s_rr[node], lane), rr0);
-      }
     }
+    push(s_rz, (double)r * (double)z);
+    push(s_rr, (double)r * (double)r);
   };
+  // A lane's slots by a tree, then a butterfly over the lanes.
   auto sum = [&](const double* s) {
-    double v = 0.0;
+    constexpr int kLane = (kDots + 31) / 32;
+    double v[kLane];
 #pragma unroll
-    for (int i = 0; i < kNodes; i += 32)
-      if (lane + i < (uint32_t)kNodes) v += s[lane + i];
-    return warp_sum_all(v);
+    for (int i = 0; i < kLane; ++i) v[i] = lane + 32 * i < (uint32_t)kDots ? s[lane + 32 * i] : 0.0;
+#pragma unroll
+    for (int n = kLane; n > 1; n = (n + 1) / 2)
+#pragma unroll
+      for (int i = 0; i < n / 2; ++i) v[i] += v[n - 1 - i];
+    return warp_sum_all(v[0]);
   };
 
   precondition();
@@ -189,13 +205,14 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
   double rz = sum(s_rz), rr = sum(s_rr);
   const LmParams& lp = d.params[P];
   const double bnorm = sqrt(rr);
-  const double stop = lp.pcg_relative_tolerance * bnorm;
+  const double stop = lp.pcg_relative_tolerance * bnorm, stop2 = stop * stop;
   const uint32_t cap = lp.max_pcg_iterations;
   uint32_t iters = 0, status = 0;
   // pcg_init (ba.wgsl:420-439): done when |b| = 0 or r.z <= 0.
   if (rr > 0.0 && rz > 0.0 && cap != 0u) {
     float beta = 0.0f;
     for (;;) {
+      const double inv_rz = inverse64(rz);
       float acc[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
       for (int j = 0; j < CPL; ++j) {
@@ -226,20 +243,14 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
       const uint32_t src = (a >= 3u ? 16u : 0u) + (part == 2u ? 8u : 0u);
       const float qu = __shfl_sync(0xffffffffu, u, src), qv = __shfl_sync(0xffffffffu, v, src);
       const float qa = own ? (part == 1u ? qv : qu) : 0.0f;
-      const double pq_node = group_sum((double)po * (double)qa);
-      if (C == 1) {
-        if (lane == 0) s_pq[node] = pq_node;
-      } else {
-        const double v0 = __shfl_sync(0xffffffffu, pq_node, 0);
-        if (lane < (uint32_t)C) st_peer(peer_addr(&s_pq[node], lane), v0);
-      }
+      push(s_pq, (double)po * (double)qa);
       team_barrier<C>();
       const double pq = sum(s_pq);
       if (!(pq > 0.0) || !isfinite(pq)) {
         status = 2;  // non-positive curvature: x unchanged
         break;
       }
-      const float alpha = (float)(rz / pq);
+      const float alpha = (float)(rz * inverse64(pq));
       x = x + alpha * po;
       r = r - alpha * qa;
       precondition();
@@ -248,7 +259,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
       const double rz_new = sum(s_rz);
       rr = sum(s_rr);
       ++iters;
-      if (sqrt(rr) <= stop || !(rz_new > 0.0)) {
+      if (rr <= stop2 || !(rz_new > 0.0)) {
         rz = rz_new;
         break;
       }
@@ -257,7 +268,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
         rz = rz_new;
         break;
       }
-      beta = (float)(rz_new / rz);
+      beta = (float)(rz_new * inv_rz);
       rz = rz_new;
     }
   }

@@ -500,9 +500,36 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
       if (small_pcg_class(P.prob_tr_begin[p + 1] - P.prob_tr_begin[p]) == k) small.push_back(p);
     d.small_off[k + 1] = (uint32_t)small.size();
   }
-  d.num_big = P.num_problems - (uint32_t)small.size();
   d.prob_tile_begin = st.up(A, tile_begin);
   d.small_list = st.up(A, small);
+  // Then the problems that fit a team of blocks; the persistent kernel has
+  // the rest.
+  const TeamPlan team = build_team_plan(P.prob_tr_begin.data(), P.num_problems, P.tile_ij, tile_begin,
+                                        (uint32_t)c->sm_count);
+  std::vector<uint8_t> big(P.num_problems, 0);
+  for (uint32_t p = 0; p < P.num_problems; ++p) {
+    big[p] = !team.in_team[p] &&
+             small_pcg_class(P.prob_tr_begin[p + 1] - P.prob_tr_begin[p]) < 0;
+    d.num_big += big[p];
+  }
+  d.prob_big = st.up(A, big);
+  d.team_rounds = team.rounds;
+  d.team_grid = team.grid;
+  d.team_smem = (uint32_t)team.smem;
+  d.team_slots_total = (uint32_t)team.cta.size();
+  d.team_cta = st.up(A, team.cta);
+  d.team_sched = st.up(A, team.sched);
+  d.team_cols = st.up(A, team.cols);
+  d.team_ents = st.up(A, team.ents);
+  if (team.rounds) {
+    // Number 0 is no exchange's.
+    const size_t words = team.z_words + 2 * kLineWords * team.cta.size();
+    d.team_z = A.alloc<unsigned long long>(words);
+    d.team_slots = d.team_z + team.z_words;
+    d.team_epoch = A.alloc<uint32_t>(P.num_problems);
+    VLBA_CUDA(cudaMemsetAsync(d.team_z, 0, 8 * words, s));
+    VLBA_CUDA(cudaMemsetAsync(d.team_epoch, 0, 4 * (size_t)P.num_problems, s));
+  }
   d.pose_prob = st.up(A, P.pose_prob);
   d.point_prob = st.up(A, P.point_prob);
   d.slot_prob = st.up(A, P.slot_prob);
@@ -778,7 +805,7 @@ void dump_trace(Context* c) {
 // the PCG kernels when the system has them.
 uint64_t iteration_launches(const Dev& d) {
   uint64_t n = 5 + (d.num_offdiag_blocks ? 1 : 0) + (d.num_long_blocks ? 1 : 0) +
-               (d.num_var_cams ? 1 : 0) + (d.num_big ? 2 : 0);
+               (d.num_var_cams ? 1 : 0) + (d.team_rounds ? 1 : 0) + (d.num_big ? 2 : 0);
   for (int k = 0; k < kSmallPcgClasses; ++k) n += d.small_off[k + 1] > d.small_off[k] ? 1 : 0;
   return n;
 }
@@ -801,7 +828,7 @@ uint64_t enqueue_iteration(Context* c, cudaEvent_t* ev) {
   check_launch(launch_offdiag(d, s), "off-diagonal blocks");
   VLBA_CUDA(cudaStreamWaitEvent(s, c->join, 0));
   if (ev) VLBA_CUDA(cudaEventRecord(ev[2], s));
-  if (c->gate && d.num_big) {
+  if (c->gate && (d.num_big || d.team_rounds)) {
     std::lock_guard<std::mutex> lock(c->gate->mu);
     VLBA_CUDA(cudaStreamWaitEvent(s, c->gate->last, 0));
     check_launch(launch_pcg(d, c->pcg_grid, s), "pcg");
