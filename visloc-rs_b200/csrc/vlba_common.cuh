@@ -107,10 +107,18 @@ struct PcgState {
   uint32_t pad;
 };
 
-// Off-diagonal blocks of at least this many terms are summed on kLongLanes
-// lanes instead of the plan's lane count (a block's summation order then
-// depends on its own length only, the same alone and in any batch).
-constexpr uint32_t kLongBlockTerms = 1024;
+// Off-diagonal blocks of at least long_block_terms terms are summed on
+// kLongLanes lanes instead of the plan's lane count (a block's summation order
+// then depends on its own length and its problem's block count only, the same
+// alone and in any batch).  Where a problem's blocks are too few to fill the
+// device at four lanes each, every block takes a warp: a lane's terms are a
+// serial chain of gathers, about 1.1 us apiece.  Measured on B200 (assembly of
+// the off-diagonal blocks, 1,024 throughout against this rule): 153 blocks of
+// 200 terms 58 -> 15 us; 48 windows in a batch 325 -> 152 us; 27,000 blocks of a
+// street 267 -> 168 us; 717,000 blocks of 39 terms keep four lanes.
+inline __host__ __device__ uint32_t long_block_terms(uint32_t problem_blocks) {
+  return problem_blocks <= 4096u ? 1u : problem_blocks <= 32768u ? 64u : 1024u;
+}
 constexpr int kLongLanes = 32;
 
 // Problems of at most this many tile rows (128 cameras) are solved by the
@@ -240,9 +248,10 @@ struct Dev {
   // (first, end) and destination, at its place in that order.
   const uint2* ord_range;      // [num_offdiag_blocks]
   const uint2* ord_dst;        // [num_offdiag_blocks]
-  // Blocks of at least kLongBlockTerms terms, summed on kLongLanes lanes
-  // (the lane count of a block follows from its own length alone), listed
-  // in any order: their term ranges and destinations, and their count.
+  // Blocks of at least their problem's prob_long_terms terms, summed on
+  // kLongLanes lanes, listed in any order: their term ranges and
+  // destinations, and their count.
+  const uint32_t* prob_long_terms;  // [num_problems] long_block_terms
   const uint2* long_range;     // [num_offdiag_blocks]
   const uint2* long_dst;       // [num_offdiag_blocks]
   uint32_t* num_long;          // [1] appended by the block order at upload

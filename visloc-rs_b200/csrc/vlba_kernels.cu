@@ -456,8 +456,8 @@ __device__ __forceinline__ void point_inverse64(const Dev& d, uint32_t l, double
 // blocks, each block's range and destination stored at its place): the groups of
 // a warp then loop about as many times (lane-pass efficiency 0.82 -> 0.99 on
 // ring-4m) while the blocks running at one time stay those of nearby rows.
-// LONG: the blocks of the long list (at least kLongBlockTerms terms) on G
-// lanes each; otherwise the other blocks in the length-sorted order.
+// LONG: the blocks of the long list (long_block_terms) on G lanes each;
+// otherwise the other blocks in the length-sorted order.
 template <int G, bool LONG>
 __global__ void __launch_bounds__(256, 2) k_offdiag(Dev d) {
   constexpr int kPerWarp = 32 / G;
@@ -480,14 +480,14 @@ __global__ void __launch_bounds__(256, 2) k_offdiag(Dev d) {
       dst = LONG ? d.long_dst[q] : d.ord_dst[q];
       c0 = range.x;
       c1 = range.y;
-      if (!LONG && c1 - c0 >= kLongBlockTerms) c1 = c0;  // the long kernel's block
       if (c0 + lane < c1) {
         pr = d.pairs[c0 + lane];
         pt = d.pair_pt[c0 + lane];
       }
       const uint32_t P =
           d.num_problems == 1 ? 0u : d.tr_prob[d.tile_ij[dst.x / tile_floats] >> 16];
-      valid = !d.ctrl[P].done && (LONG || range.y - range.x < kLongBlockTerms);
+      valid = !d.ctrl[P].done;
+      if (!LONG && c1 - c0 >= d.prob_long_terms[P]) valid = false;  // the long kernel's block
     }
     float acc[36], cmp[36];
 #pragma unroll
@@ -2214,10 +2214,11 @@ __global__ void k_wait_probe(const unsigned int* flag, unsigned long long limit_
 // ties in plan order (a block's rank is the count of blocks of its window
 // before it in that order); each block's term range and destination are
 // written at its place in that order.
-__global__ void __launch_bounds__(256) k_block_order(const uint32_t* blk_off, const uint2* blk_dst,
-                                                     uint32_t nb, uint32_t g, uint2* ord_range,
-                                                     uint2* ord_dst, uint2* long_range,
-                                                     uint2* long_dst, uint32_t* num_long) {
+__global__ void __launch_bounds__(256) k_block_order(Dev d, uint2* ord_range, uint2* ord_dst,
+                                                     uint2* long_range, uint2* long_dst) {
+  const uint32_t* const blk_off = d.blk_off;
+  const uint2* const blk_dst = d.blk_dst;
+  const uint32_t nb = d.num_offdiag_blocks, g = d.group;
   __shared__ uint32_t key[256];
   const uint32_t b0 = blockIdx.x * 256u, t = threadIdx.x;
   const uint32_t n = min(256u, nb - b0);
@@ -2234,8 +2235,11 @@ __global__ void __launch_bounds__(256) k_block_order(const uint32_t* blk_off, co
     const uint2 range = make_uint2(blk_off[b0 + t], blk_off[b0 + t + 1]);
     ord_range[b0 + rank] = range;
     ord_dst[b0 + rank] = blk_dst[b0 + t];
-    if (range.y - range.x >= kLongBlockTerms) {
-      const uint32_t at = atomicAdd(num_long, 1u);  // any order: a block's sums do not depend on it
+    const uint32_t P = d.num_problems == 1
+                           ? 0u
+                           : d.tr_prob[d.tile_ij[blk_dst[b0 + t].x / (d.tb * d.tb * kBlock)] >> 16];
+    if (range.y - range.x >= d.prob_long_terms[P]) {
+      const uint32_t at = atomicAdd(d.num_long, 1u);  // any order: a block's sums do not depend on it
       long_range[at] = range;
       long_dst[at] = blk_dst[b0 + t];
     }
@@ -2346,18 +2350,20 @@ cudaError_t launch_point_prep(const Dev& d, cudaStream_t s) {
 
 cudaError_t launch_offdiag(const Dev& d, cudaStream_t s) {
   if (d.num_offdiag_blocks == 0) return cudaSuccess;
-  const size_t threads_needed = (size_t)d.num_offdiag_blocks * d.group;
-  const int g = grid1d(threads_needed, 256, 148 * 16);
-  switch (d.group) {
-    case 1: k_offdiag<1, false><<<g, 256, 0, s>>>(d); break;
-    case 2: k_offdiag<2, false><<<g, 256, 0, s>>>(d); break;
-    case 4: k_offdiag<4, false><<<g, 256, 0, s>>>(d); break;
-    case 8: k_offdiag<8, false><<<g, 256, 0, s>>>(d); break;
-    case 16: k_offdiag<16, false><<<g, 256, 0, s>>>(d); break;
-    default: k_offdiag<32, false><<<g, 256, 0, s>>>(d); break;
+  if (d.num_long_blocks < d.num_offdiag_blocks) {  // else every block is on the long list
+    const size_t threads_needed = (size_t)d.num_offdiag_blocks * d.group;
+    const int g = grid1d(threads_needed, 256, 148 * 16);
+    switch (d.group) {
+      case 1: k_offdiag<1, false><<<g, 256, 0, s>>>(d); break;
+      case 2: k_offdiag<2, false><<<g, 256, 0, s>>>(d); break;
+      case 4: k_offdiag<4, false><<<g, 256, 0, s>>>(d); break;
+      case 8: k_offdiag<8, false><<<g, 256, 0, s>>>(d); break;
+      case 16: k_offdiag<16, false><<<g, 256, 0, s>>>(d); break;
+      default: k_offdiag<32, false><<<g, 256, 0, s>>>(d); break;
+    }
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
   }
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
   if (d.num_long_blocks == 0) return cudaSuccess;
   const int gl = grid1d((size_t)d.num_long_blocks * kLongLanes, 256, 148 * 16);
   k_offdiag<kLongLanes, true><<<gl, 256, 0, s>>>(d);
@@ -2448,9 +2454,8 @@ cudaError_t launch_block_order(const Dev& d, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(d.num_long, 0, 4, s);
   if (e != cudaSuccess) return e;
   k_block_order<<<(d.num_offdiag_blocks + 255) / 256, 256, 0, s>>>(
-      d.blk_off, d.blk_dst, d.num_offdiag_blocks, d.group, const_cast<uint2*>(d.ord_range),
-      const_cast<uint2*>(d.ord_dst), const_cast<uint2*>(d.long_range),
-      const_cast<uint2*>(d.long_dst), d.num_long);
+      d, const_cast<uint2*>(d.ord_range), const_cast<uint2*>(d.ord_dst),
+      const_cast<uint2*>(d.long_range), const_cast<uint2*>(d.long_dst));
   return cudaGetLastError();
 }
 

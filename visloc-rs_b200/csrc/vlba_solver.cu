@@ -513,6 +513,15 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
     d.num_big += big[p];
   }
   d.prob_big = st.up(A, big);
+  std::vector<uint32_t> long_terms(P.num_problems, 0u);  // blocks, then the threshold
+  if (P.num_problems == 1) {
+    long_terms[0] = (uint32_t)P.blk_dst.size();
+  } else {
+    const uint32_t tf = P.tb * P.tb * kBlock;
+    for (const PairIdx& b : P.blk_dst) ++long_terms[P.tile_meta[4 * (size_t)(b.a / tf) + 3]];
+  }
+  for (uint32_t& n : long_terms) n = long_block_terms(n);
+  d.prob_long_terms = st.up(A, long_terms);
   d.team_rounds = team.rounds;
   d.team_grid = team.grid;
   d.team_smem = (uint32_t)team.smem;
@@ -804,7 +813,7 @@ void dump_trace(Context* c) {
 // decide always; off-diagonal (short and long blocks), camera-diagonal and
 // the PCG kernels when the system has them.
 uint64_t iteration_launches(const Dev& d) {
-  uint64_t n = 5 + (d.num_offdiag_blocks ? 1 : 0) + (d.num_long_blocks ? 1 : 0) +
+  uint64_t n = 5 + (d.num_offdiag_blocks > d.num_long_blocks ? 1 : 0) + (d.num_long_blocks ? 1 : 0) +
                (d.num_var_cams ? 1 : 0) + (d.team_rounds ? 1 : 0) + (d.num_big ? 2 : 0);
   for (int k = 0; k < kSmallPcgClasses; ++k) n += d.small_off[k + 1] > d.small_off[k] ? 1 : 0;
   return n;
