@@ -674,6 +674,46 @@ __device__ __forceinline__ void cam_diag_obs(const Dev& d, uint32_t k, uint32_t 
   acc[26] += X * w[1] - Y * w[0];
 }
 
+// One column of the inverse of the SPD matrix whose upper triangle is u[21], by
+// Cholesky in FP64 registers: every lane factors (a chain of six reciprocal
+// square roots and no divisions), lane c keeps column c % 6.  False (for every
+// lane) if the matrix is not positive definite.
+__device__ __forceinline__ bool chol_column6(const double* u, uint32_t c, double (&x)[6]) {
+  double L[6][6], il[6];
+  bool ok = true;
+#pragma unroll
+  for (int j = 0; j < 6; ++j) {
+    double s = u[ut6(j, j)];
+#pragma unroll
+    for (int q = 0; q < j; ++q) s = fma(-L[j][q], L[j][q], s);
+    ok = ok && s > 0.0 && isfinite(s);
+    il[j] = rsqrt(s);
+#pragma unroll
+    for (int i = j + 1; i < 6; ++i) {
+      double t = u[ut6(j, i)];
+#pragma unroll
+      for (int q = 0; q < j; ++q) t = fma(-L[i][q], L[j][q], t);
+      L[i][j] = t * il[j];
+    }
+  }
+  double y[6];
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {
+    double s = c % 6u == (uint32_t)i ? 1.0 : 0.0;
+#pragma unroll
+    for (int q = 0; q < i; ++q) s = fma(-L[i][q], y[q], s);
+    y[i] = s * il[i];
+  }
+#pragma unroll
+  for (int i = 5; i >= 0; --i) {
+    double s = y[i];
+#pragma unroll
+    for (int q = i + 1; q < 6; ++q) s = fma(-L[q][i], x[q], s);
+    x[i] = s * il[i];
+  }
+  return ok;
+}
+
 __global__ void __launch_bounds__(kDiagThreads) k_cam_diag(Dev d) {
   __shared__ double red[(kDiagThreads / 32) * kDiagAcc];
   __shared__ double tot[kDiagAcc];
@@ -727,21 +767,29 @@ __global__ void __launch_bounds__(kDiagThreads) k_cam_diag(Dev d) {
     }
     diag_block_sum<kDiagAcc>(acc, red, tot);
     const double lambda = d.ctrl[P].lambda;
-    if (t == 0) {
-      double S[36], inv[36];
+    // Warp 0 writes the block and its inverse, a column per lane (by one
+    // thread, with the divisions of a textbook factorisation, this tail took 10
+    // of the kernel's 25 us on a 20-camera window).
+    if (t < 32) {
+      double u[21];
+#pragma unroll
       for (int r = 0; r < 6; ++r)
-        for (int cc = 0; cc < 6; ++cc) {
-          double v = r <= cc ? tot[ut6(r, cc)] : tot[ut6(cc, r)];
-          if (r == cc && lambda > 0.0) v += lambda;
-          S[r * 6 + cc] = v;
-        }
+#pragma unroll
+        for (int cc = r; cc < 6; ++cc)
+          u[ut6(r, cc)] = tot[ut6(r, cc)] + (r == cc && lambda > 0.0 ? lambda : 0.0);
       float* blk = d.tiles + d.diag_dst[s];
-      for (int e = 0; e < 36; ++e) blk[e] = (float)S[e];
-      for (int a = 0; a < 6; ++a) d.rhs[6 * (size_t)s + a] = (float)tot[21 + a];
-      const bool ok = chol_inverse6(S, inv);
-      if (ok)
-        for (int e = 0; e < 36; ++e) d.minv[36 * (size_t)s + e] = (float)inv[e];
-      s_fail = ok ? 0 : 1;
+      for (uint32_t e = t; e < 36; e += 32) {
+        const uint32_t r = e / 6, cc = e % 6;
+        blk[e] = (float)(tot[r <= cc ? ut6(r, cc) : ut6(cc, r)] +
+                         (r == cc && lambda > 0.0 ? lambda : 0.0));
+      }
+      if (t < 6) d.rhs[6 * (size_t)s + t] = (float)tot[21 + t];
+      double col[6];
+      const bool ok = chol_column6(u, t, col);
+      if (ok && t < 6)
+#pragma unroll
+        for (int a = 0; a < 6; ++a) d.minv[36 * (size_t)s + a * 6 + t] = (float)col[a];
+      if (t == 0) s_fail = ok ? 0 : 1;
     }
     __syncthreads();
     if (s_fail) {
