@@ -281,7 +281,9 @@ struct Dev {
   uint32_t l2_resident_tiles;  // tiles [0, n) are streamed with L2 evict_last
   unsigned int* barrier;       // [kBarrierWords]: [0] grid-barrier arrivals, [2] active problems
                                // problems, -, group counts
-  unsigned int* error;         // [1] device error flags
+  unsigned int* error;         // [2] device error flags; problems done
+  unsigned int* host_state;    // page-locked host memory: [0] every problem is done, [1] error
+                               // flags, both as of the last k_decide
   // Optional PCG phase trace (globaltimer ns): [iteration][block][kTracePhases]
   // for iterations < kTraceIters; null unless VLBA_TRACE_PCG is set.
   unsigned long long* trace;

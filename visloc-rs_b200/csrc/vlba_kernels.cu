@@ -1085,9 +1085,16 @@ __global__ void __launch_bounds__(256) k_decide(Dev d) {
   __shared__ unsigned long long redu[256];
   const uint32_t P = blockIdx.x;
   if (P >= d.num_problems) return;
+  if (P == 0 && threadIdx.x == 0) d.host_state[1] = *(volatile unsigned int*)d.error;
   Ctrl& c = d.ctrl[P];
   if (c.done) return;
   const LmParams& lp = d.params[P];
+  // The problem is done; the last one tells the host (which looks once this
+  // kernel has finished).
+  auto finish = [&]() {
+    c.done = 1u;
+    if (atomicAdd(d.error + 1, 1u) + 1u == d.num_problems) d.host_state[0] = 1u;
+  };
   double cost = 0.0, lstep = 0.0, pstep = 0.0;
   unsigned long long bad = 0;
   for (uint32_t ch = d.prob_chunk_begin[P] + threadIdx.x; ch < d.prob_chunk_begin[P + 1];
@@ -1116,7 +1123,7 @@ __global__ void __launch_bounds__(256) k_decide(Dev d) {
     c.converged = 0u;
     c.nonfinite = 0u;
     c.total_pcg = 0ull;
-    if (lp.max_iterations == 0) c.done = 1u;
+    if (lp.max_iterations == 0) finish();
     return;
   }
   const uint32_t it = c.iteration;
@@ -1188,7 +1195,7 @@ __global__ void __launch_bounds__(256) k_decide(Dev d) {
   c.iteration = it + 1;
   c.relinearize = accepted ? 1u : 0u;
   c.nonfinite = 0u;
-  if (stop || c.iteration >= lp.max_iterations) c.done = 1u;
+  if (stop || c.iteration >= lp.max_iterations) finish();
 }
 
 // -------------------------------------------------------------------- PCG

@@ -2,7 +2,8 @@
 // of include/visloc_ba_cuda.h.
 //
 // The LM loop runs on the device (k_decide owns accept/reject and lambda);
-// the host only issues the per-iteration kernel sequence and polls a 4-byte
+// the host only issues the per-iteration kernel sequence, one iteration ahead
+// of the device, and looks at a 4-byte
 // "all done" word per iteration.  The reference's host loop instead reads
 // back the step and evaluates the cost on the CPU every iteration
 // (crates/ba-gpu/src/solver.rs:514-548, 696-727).
@@ -199,6 +200,8 @@ struct Context {
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
   cudaEvent_t ev[6] = {};
+  cudaEvent_t step_ev[2] = {};     // the ends of the last two LM iterations issued
+  unsigned int* host_state = nullptr;  // Dev::host_state
   std::string error;
   Arena arena;
   Plan plan;
@@ -644,9 +647,10 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
     d.trace = A.alloc<unsigned long long>((size_t)kTraceIters * c->pcg_grid_hint *
                                           (kTracePhases + 2 * 32 + 32 * 8 * 4));
   d.barrier = A.alloc<unsigned int>(kBarrierWords);
-  d.error = A.alloc<unsigned int>(1);
+  d.error = A.alloc<unsigned int>(2);
+  d.host_state = c->host_state;
   VLBA_CUDA(cudaMemsetAsync(d.barrier, 0, 4 * kBarrierWords, s));
-  VLBA_CUDA(cudaMemsetAsync(d.error, 0, 4, s));
+  VLBA_CUDA(cudaMemsetAsync(d.error, 0, 8, s));
   d.chunk_point_begin = st.up(A, P.chunk_point_begin);
   const size_t nch = P.chunk_point_begin.size() - 1;
   d.chunk_cost = A.alloc<double>(nch);
@@ -745,7 +749,7 @@ void reset_state(Context* c) {
   VLBA_CUDA(cudaMemcpyAsync(d.pose_t[0], d.init_pose_t, P.pose_t.size() * 8, cudaMemcpyDeviceToDevice, s));
   VLBA_CUDA(cudaMemcpyAsync(d.points[0], d.init_points, P.points.size() * 8, cudaMemcpyDeviceToDevice, s));
   VLBA_CUDA(cudaMemsetAsync(d.ctrl, 0, sizeof(Ctrl) * P.num_problems, s));
-  VLBA_CUDA(cudaMemsetAsync(d.error, 0, 4, s));
+  VLBA_CUDA(cudaMemsetAsync(d.error, 0, 8, s));
 }
 
 
@@ -931,16 +935,30 @@ RunStats run_lm(Context* c, bool profile, PhaseTimes* pt) {
   for (const LmParams& lp : c->plan.params) max_iters = std::max(max_iters, lp.max_iterations);
   if ((c->flags & VLBA_FLAG_GRAPH) && !profile && !d.trace) return run_lm_graph(c, max_iters);
   RunStats st;
-  std::vector<Ctrl> ctrl(c->plan.num_problems);
+  volatile unsigned int* const state = c->host_state;  // written by k_decide
+  state[0] = state[1] = 0u;
+  auto check_error = [&] {
+    if (const unsigned int err = state[1]) {
+      VLBA_CUDA(cudaStreamSynchronize(s));
+      throw Status(VLBA_ERR_TIMEOUT,
+                   "a bounded device wait gave up (error bits " + std::to_string(err) + ")");
+    }
+  };
   VLBA_CUDA(cudaEventRecord(c->ev[0], s));
   st.launches += enqueue_initial(c);
+  // One iteration is issued ahead of the one whose end is awaited, so the
+  // device never waits for the host between two; the one in flight when the
+  // last problem finishes finds nothing to do.
+  const bool step = profile || d.trace;
   for (uint32_t it = 0; it < max_iters; ++it) {
     st.launches += enqueue_iteration(c, profile ? c->ev + 1 : nullptr);
-    // Poll the per-problem control words (one small copy per iteration).
-    VLBA_CUDA(cudaMemcpyAsync(ctrl.data(), d.ctrl, sizeof(Ctrl) * ctrl.size(), cudaMemcpyDeviceToHost, s));
-    unsigned int err = 0;
-    VLBA_CUDA(cudaMemcpyAsync(&err, d.error, 4, cudaMemcpyDeviceToHost, s));
-    VLBA_CUDA(cudaStreamSynchronize(s));
+    VLBA_CUDA(cudaEventRecord(c->step_ev[it & 1], s));
+    if (step) {
+      VLBA_CUDA(cudaEventSynchronize(c->step_ev[it & 1]));
+    } else {
+      if (it == 0) continue;
+      VLBA_CUDA(cudaEventSynchronize(c->step_ev[(it - 1) & 1]));
+    }
     if (profile) {
       float a = 0.f, b = 0.f, e = 0.f, f = 0.f;
       VLBA_CUDA(cudaEventElapsedTime(&a, c->ev[1], c->ev[2]));
@@ -952,13 +970,12 @@ RunStats run_lm(Context* c, bool profile, PhaseTimes* pt) {
       pt->pcg.push_back(e);
       pt->update.push_back(f);
     }
-    if (err) throw Status(VLBA_ERR_TIMEOUT, "a bounded device wait gave up (error bits " + std::to_string(err) + ")");
-    bool all_done = true;
-    for (const Ctrl& x : ctrl) all_done = all_done && x.done;
-    if (all_done) break;
+    check_error();
+    if (state[0]) break;
   }
   VLBA_CUDA(cudaEventRecord(c->ev[5], s));
   VLBA_CUDA(cudaEventSynchronize(c->ev[5]));
+  check_error();
   float ms = 0.f;
   VLBA_CUDA(cudaEventElapsedTime(&ms, c->ev[0], c->ev[5]));
   st.device_ms = ms;
@@ -1418,6 +1435,9 @@ Context* make_context(int device) {
   VLBA_CUDA(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
   VLBA_CUDA(cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming));
   for (auto& e : c->ev) VLBA_CUDA(cudaEventCreate(&e));
+  for (auto& e : c->step_ev) VLBA_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  VLBA_CUDA(cudaHostAlloc(&c->host_state, 2 * sizeof(unsigned int), cudaHostAllocMapped));
+  c->host_state[0] = c->host_state[1] = 0u;
   return c.release();
 }
 
@@ -1428,6 +1448,9 @@ void free_context(Context* c) {
   c->arena.release();
   for (auto& e : c->ev)
     if (e) cudaEventDestroy(e);
+  for (auto& e : c->step_ev)
+    if (e) cudaEventDestroy(e);
+  if (c->host_state) cudaFreeHost(c->host_state);
   for (int i = 0; i < 2; ++i) {
     if (c->stage_ev[i]) cudaEventDestroy(c->stage_ev[i]);
     if (c->stage[i]) cudaFreeHost(c->stage[i]);
