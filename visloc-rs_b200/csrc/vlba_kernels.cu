@@ -91,33 +91,42 @@ __device__ __forceinline__ void btkb(const T* K, T x, T y, T z, T* out) {
   }
 }
 
-// Fixed-order block reductions (deterministic for a given block size).
-template <typename T, int N>
-__device__ __forceinline__ T block_sum(T v, T* red) {
-  red[threadIdx.x] = v;
-  __syncthreads();
+// Fixed-order sums of cost and bad and the maxima of step and (TWO) step2 over
+// a block of 256 threads, in thread 0: a butterfly within each warp, then the
+// warps in order.  `red` is free again once every thread has passed the
+// second barrier.
+struct CostReduction {
+  double cost[8], step[8], step2[8];
+  unsigned long long bad[8];
+};
+template <bool TWO>
+__device__ __forceinline__ void reduce_cost(double& cost, unsigned long long& bad, double& step,
+                                            double& step2, CostReduction& red) {
 #pragma unroll
-  for (int s = N / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
+  for (int off = 16; off > 0; off >>= 1) {
+    cost += __shfl_xor_sync(0xffffffffu, cost, off);
+    bad += __shfl_xor_sync(0xffffffffu, bad, off);
+    step = fmax(step, __shfl_xor_sync(0xffffffffu, step, off));
+    if (TWO) step2 = fmax(step2, __shfl_xor_sync(0xffffffffu, step2, off));
   }
-  const T out = red[0];
+  const uint32_t warp = threadIdx.x >> 5;
+  if ((threadIdx.x & 31u) == 0) {
+    red.cost[warp] = cost;
+    red.bad[warp] = bad;
+    red.step[warp] = step;
+    if (TWO) red.step2[warp] = step2;
+  }
   __syncthreads();
-  return out;
-}
-
-template <int N>
-__device__ __forceinline__ double block_max(double v, double* red) {
-  red[threadIdx.x] = v;
-  __syncthreads();
+  if (threadIdx.x == 0) {
 #pragma unroll
-  for (int s = N / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + s]);
-    __syncthreads();
+    for (int w = 1; w < 8; ++w) {
+      cost += red.cost[w];
+      bad += red.bad[w];
+      step = fmax(step, red.step[w]);
+      if (TWO) step2 = fmax(step2, red.step2[w]);
+    }
   }
-  const double out = red[0];
   __syncthreads();
-  return out;
 }
 
 // 6x6 SPD inverse by Cholesky in FP64; false if not positive definite.
@@ -922,8 +931,7 @@ __global__ void __launch_bounds__(256) k_pose_update(Dev d) {
 // Sums in a fixed order per chunk.
 template <bool TRIAL>
 __global__ void __launch_bounds__(256) k_cost(Dev d) {
-  __shared__ double red[256];
-  __shared__ unsigned long long redu[256];
+  __shared__ CostReduction red;
   __shared__ double sX[3 * 256];                      // the chunk's (candidate) points
   __shared__ float sXf[TRIAL ? 3 * 256 : 1];          // the points as FP32 (pt_s)
   __shared__ double sC[TRIAL ? 3 * kObsStage : 1];    // staged observation terms
@@ -1062,13 +1070,12 @@ __global__ void __launch_bounds__(256) k_cost(Dev d) {
       const double rc = robust_cost(lp.robust_kernel, lp.robust_parameter, ss);
       cost += d.obs_w ? d.obs_w[k] * rc : rc;  // w * rho(s) (problem.rs:497-560)
     }
-    const double tc = block_sum<double, 256>(cost, red);
-    const unsigned long long tb = block_sum<unsigned long long, 256>(bad, redu);
-    const double ts = block_max<256>(step, red);
+    double none = 0.0;
+    reduce_cost<false>(cost, bad, step, none, red);
     if (threadIdx.x == 0) {
-      d.chunk_cost[ch] = tc;
-      d.chunk_bad[ch] = tb;
-      d.chunk_step[ch] = ts;
+      d.chunk_cost[ch] = cost;
+      d.chunk_bad[ch] = bad;
+      d.chunk_step[ch] = step;
     }
   }
 }
@@ -1081,8 +1088,7 @@ __global__ void __launch_bounds__(256) k_cost(Dev d) {
 // A non-finite step is the reference's SingularSystem: lambda up, no step.
 template <bool INIT>
 __global__ void __launch_bounds__(256) k_decide(Dev d) {
-  __shared__ double red[256];
-  __shared__ unsigned long long redu[256];
+  __shared__ CostReduction red;
   const uint32_t P = blockIdx.x;
   if (P >= d.num_problems) return;
   if (P == 0 && threadIdx.x == 0) d.host_state[1] = *(volatile unsigned int*)d.error;
@@ -1107,10 +1113,7 @@ __global__ void __launch_bounds__(256) k_decide(Dev d) {
     for (uint32_t p = d.prob_pose_begin[P] + threadIdx.x; p < d.prob_pose_begin[P + 1];
          p += blockDim.x)
       pstep = fmax(pstep, d.pose_step[p]);
-  cost = block_sum<double, 256>(cost, red);
-  bad = block_sum<unsigned long long, 256>(bad, redu);
-  lstep = block_max<256>(lstep, red);
-  pstep = block_max<256>(pstep, red);
+  reduce_cost<true>(cost, bad, lstep, pstep, red);
   if (threadIdx.x != 0) return;
   if (INIT) {
     c.initial_cost = cost;
