@@ -8,8 +8,9 @@
 // solve and an iteration crosses two barriers of one cluster (of one block
 // for up to 16 cameras), the same recurrence and stopping rule:
 //
-//   one warp per camera: lane l holds columns l, l + 32, ... of the camera's
-//   six rows of S, and its own copy of those entries of p;
+//   one warp per camera (two of 17 to 32 cameras): lane l holds columns l,
+//   l + 32, ... of the camera's six rows of S, and its own copy of those
+//   entries of p;
 //   q = S p      each lane's partial products, then a reduce-scatter butterfly
 //   -- barrier: every warp's p.q
 //   x, r, z of the camera on lanes 0-5; z pushed to every block of the
@@ -18,13 +19,14 @@
 //   p = z + beta p, on every lane for its columns.
 //
 // What bounds it is the chain of one iteration (LDS, FMA, shuffles, barrier),
-// so the cluster is as small as the registers allow: 3 columns per lane up to
-// 16 cameras (one block), 6 up to 32 (two), 12 up to 64 (four blocks of 16
-// warps, 72 registers of S per thread) and 24 up to 128 (sixteen blocks of 8
-// warps, 144 registers).  Whole LM solves from host arrays on B200, k_pcg
-// against this kernel: a 20-keyframe window (10 LM iterations) 5.19 -> 2.90
-// ms, 50 cameras (20) 9.9 -> 5.3 ms, GNC on 60 cameras 31.7 -> 19.4 ms, 48
-// windows in one batch (6) 8.35 -> 6.27 ms.
+// so the cluster is as small as the registers allow (a cluster's barrier takes
+// 330 cycles and more, a block's 20): one block of 16 warps up to 16 cameras (3
+// columns per lane) and up to 32 (6 columns, two cameras a warp), four blocks
+// up to 64 (12 columns, 72 registers of S per thread) and sixteen blocks of 8
+// warps up to 128 (24 columns, 144 registers).  Measured on B200 for one LM
+// iteration's solve, k_pcg against this kernel: 18 cameras and 29 PCG
+// iterations 300 -> 42 us, 48 cameras and 25 iterations 280 -> 60 us, a batch
+// of 48 windows of up to 36 cameras 554 -> 167 us over its three classes.
 //
 // Every sum runs in an order fixed by the problem's own size, so a problem
 // solves the same alone and in any batch.  The cluster's blocks compute the
@@ -79,28 +81,29 @@ __device__ __forceinline__ void team_barrier() {
   }
 }
 
-// C blocks of W warps, one camera per warp; CPL columns of S per lane
-// (32 CPL = 6 C W).
-template <int C, int W, int CPL>
+// C blocks of W warps, N cameras per warp; CPL columns of S per lane
+// (32 CPL = 6 C W N).
+template <int C, int W, int CPL, int N>
 __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* list) {
-  constexpr int kNodes = C * W, kRows = kNodes / 8;
+  constexpr int kNodes = C * W * N, kRows = kNodes / 8;
   // Dot slots of a camera: its six products (a warp then sums them all, three
   // butterfly levels fewer in the chain), or one sum where six would be more
   // to push to every block than that saves (four blocks: 91 us a solve of 40
   // cameras with sums, 106 with products).
-  constexpr int kPer = C <= 2 ? 6 : 1, kDots = kPer * kNodes;
+  constexpr int kPer = C == 1 ? 6 : 1, kDots = kPer * kNodes;
+  static_assert(C == 1 || N == 1, "a camera a warp where blocks exchange");
   static_assert(32 * CPL == 6 * kNodes, "a lane's columns cover the system");
   __shared__ float zs[32 * CPL];
   __shared__ double s_pq[kDots], s_rz[kDots], s_rr[kDots];
+  __shared__ double s_sum[2];
   __shared__ uint32_t tmap[kRows * kRows];  // tile of (I, J), J <= I
   const uint32_t P = list[blockIdx.x / C];
   if (d.ctrl[P].done) return;  // the same for every block of the cluster
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t rank = C == 1 ? 0u : blockIdx.x % C;
-  const uint32_t node = rank * W + warp;
+  const uint32_t node = (rank * W + warp) * N;  // the warp's first camera
   const uint32_t tr0 = d.prob_tr_begin[P], rows = d.prob_tr_begin[P + 1] - tr0;
   const uint32_t nodes = rows * 8u;  // padded slots have zero rows and rhs
-  const bool mine = node < nodes;
 
   for (uint32_t i = threadIdx.x; i < (uint32_t)(kRows * kRows); i += 32 * W) tmap[i] = kNone;
   __syncthreads();
@@ -110,43 +113,48 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
   }
   __syncthreads();
 
-  // The camera's six rows of S: from the tile right of (or on) the diagonal
-  // of its tile row, else the mirrored block of the lower tile.
-  float S[6][CPL], p[CPL];
+  // The cameras' rows of S: from the tile right of (or on) the diagonal of
+  // its tile row, else the mirrored block of the lower tile.
+  float S[N][6][CPL], p[CPL];
 #pragma unroll
   for (int j = 0; j < CPL; ++j) {
     const uint32_t col = lane + 32u * j, cn = col / 6u, c = col % 6u;
     p[j] = 0.0f;
 #pragma unroll
-    for (int r = 0; r < 6; ++r) S[r][j] = 0.0f;
-    if (mine && cn < nodes) {
-      const uint32_t I = node >> 3, J = cn >> 3;
-      const bool lower = I >= J;
-      const uint32_t t = lower ? tmap[I * kRows + J] : tmap[J * kRows + I];
-      if (t != kNone) {
-        const float* tile = d.tiles + (size_t)t * (64 * kBlock);
-        if (lower) {
-          const float* b = tile + ((node & 7u) * 8u + (cn & 7u)) * kBlock + c;
+    for (int u = 0; u < N; ++u) {
 #pragma unroll
-          for (int r = 0; r < 6; ++r) S[r][j] = b[6 * r];
-        } else {
-          const float2* b =
-              reinterpret_cast<const float2*>(tile + ((cn & 7u) * 8u + (node & 7u)) * kBlock + c * 6u);
+      for (int r = 0; r < 6; ++r) S[u][r][j] = 0.0f;
+      const uint32_t n = node + u;
+      if (n < nodes && cn < nodes) {
+        const uint32_t I = n >> 3, J = cn >> 3;
+        const bool lower = I >= J;
+        const uint32_t t = lower ? tmap[I * kRows + J] : tmap[J * kRows + I];
+        if (t != kNone) {
+          const float* tile = d.tiles + (size_t)t * (64 * kBlock);
+          if (lower) {
+            const float* b = tile + ((n & 7u) * 8u + (cn & 7u)) * kBlock + c;
 #pragma unroll
-          for (int r = 0; r < 3; ++r) {
-            const float2 v = b[r];
-            S[2 * r][j] = v.x;
-            S[2 * r + 1][j] = v.y;
+            for (int r = 0; r < 6; ++r) S[u][r][j] = b[6 * r];
+          } else {
+            const float2* b =
+                reinterpret_cast<const float2*>(tile + ((cn & 7u) * 8u + (n & 7u)) * kBlock + c * 6u);
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+              const float2 v = b[r];
+              S[u][2 * r][j] = v.x;
+              S[u][2 * r + 1][j] = v.y;
+            }
           }
         }
       }
     }
   }
 
-  // The camera's vector entries on lanes 0-5 (zero on the others).
-  const uint32_t a = lane < 6u ? lane : 0u;
-  const bool own = mine && lane < 6u;
-  const size_t at = (size_t)6 * (8u * tr0 + node) + a;
+  // The cameras' vector entries on lanes 0 to 6 N - 1 (zero on the others):
+  // entry a of the warp's camera `sub`.
+  const uint32_t sub = lane < 6u * N ? lane / 6u : 0u, a = lane < 6u * N ? lane % 6u : 0u;
+  const bool own = node + sub < nodes && lane < 6u * N;
+  const size_t at = (size_t)6 * (8u * tr0 + node + sub) + a;
   float m[6];
 #pragma unroll
   for (int b = 0; b < 6; ++b) m[b] = own ? d.minv[6 * at + b] : 0.0f;
@@ -154,13 +162,13 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
   auto precondition = [&]() {
     z = 0.0f;
 #pragma unroll
-    for (int b = 0; b < 6; ++b) z += m[b] * __shfl_sync(0xffffffffu, r, b);
+    for (int b = 0; b < 6; ++b) z += m[b] * __shfl_sync(0xffffffffu, r, 6u * sub + b);
   };
   // The camera's products v (lanes 0-5) into its slots of every block.
   auto push = [&](double* slots, double v) {
     if (kPer == 1) v = group_sum(v);
     if (C == 1) {
-      if (lane < (uint32_t)kPer) slots[kPer * node + lane] = v;
+      if (lane < (uint32_t)(kPer * N)) slots[kPer * node + lane] = v;
     } else {
 #pragma unroll
       for (int i = 0; i < kPer * C; i += 32) {
@@ -173,7 +181,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
   // z and the products of r.z and r.r into every block of the cluster.
   auto publish = [&]() {
     if (C == 1) {
-      if (lane < 6u) zs[6 * node + lane] = z;
+      if (lane < 6u * N) zs[6 * node + lane] = z;
     } else {
 #pragma unroll
       for (int i = 0; i < 6 * C; i += 32) {
@@ -197,12 +205,23 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
       for (int i = 0; i < n / 2; ++i) v[i] += v[n - 1 - i];
     return warp_sum_all(v[0]);
   };
+  // The sums every thread of the block needs, each by one warp: with all
+  // sixteen summing for themselves the shuffle unit was the bound.
+  auto totals = [&](const double* s0, const double* s1) {
+    if (warp < 2 && (warp == 0 || s1)) {
+      const double v = sum(warp == 0 ? s0 : s1);
+      if (lane == 0) s_sum[warp] = v;
+    }
+    __syncthreads();
+    return make_double2(s_sum[0], s_sum[1]);
+  };
 
   precondition();
   if (C > 1) team_barrier<C>();  // every block runs before its memory is written
   publish();
   team_barrier<C>();
-  double rz = sum(s_rz), rr = sum(s_rr);
+  const double2 first = totals(s_rz, s_rr);
+  double rz = first.x, rr = first.y;
   const LmParams& lp = d.params[P];
   const double bnorm = sqrt(rr);
   const double stop = lp.pcg_relative_tolerance * bnorm, stop2 = stop * stop;
@@ -213,39 +232,50 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
     float beta = 0.0f;
     for (;;) {
       const double inv_rz = inverse64(rz);
-      float acc[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+      float acc[N][6];
+#pragma unroll
+      for (int u = 0; u < N; ++u)
+#pragma unroll
+        for (int q = 0; q < 6; ++q) acc[u][q] = 0.0f;
 #pragma unroll
       for (int j = 0; j < CPL; ++j) {
         p[j] = __fmaf_rn(beta, p[j], zs[lane + 32 * j]);
 #pragma unroll
-        for (int q = 0; q < 6; ++q) acc[q] = __fmaf_rn(S[q][j], p[j], acc[q]);
+        for (int u = 0; u < N; ++u)
+#pragma unroll
+          for (int q = 0; q < 6; ++q) acc[u][q] = __fmaf_rn(S[u][q][j], p[j], acc[u][q]);
       }
       po = __fmaf_rn(beta, po, z);
       // Row sums over the lanes: a reduce-scatter (bit 4 keeps three of the
       // six rows, bit 3 two or one of those), then a butterfly; then row a
-      // back to lane a.
+      // back to its lane.
       const bool b4 = (lane >> 4) & 1u, b3 = (lane >> 3) & 1u;
-      float h[3];
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        const float keep = b4 ? acc[q + 3] : acc[q], send = b4 ? acc[q] : acc[q + 3];
-        h[q] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-      }
-      const float g0 = __shfl_xor_sync(0xffffffffu, b3 ? h[0] : h[2], 8);
-      const float g1 = __shfl_xor_sync(0xffffffffu, h[1], 8);
-      float u = b3 ? h[2] + g0 : h[0] + g0, v = h[1] + g1;  // v: rows 1 and 4, where b3 is 0
-#pragma unroll
-      for (int off = 4; off > 0; off >>= 1) {
-        u += __shfl_xor_sync(0xffffffffu, u, off);
-        v += __shfl_xor_sync(0xffffffffu, v, off);
-      }
       const uint32_t part = a >= 3u ? a - 3u : a;
       const uint32_t src = (a >= 3u ? 16u : 0u) + (part == 2u ? 8u : 0u);
-      const float qu = __shfl_sync(0xffffffffu, u, src), qv = __shfl_sync(0xffffffffu, v, src);
-      const float qa = own ? (part == 1u ? qv : qu) : 0.0f;
+      float qa = 0.0f;
+#pragma unroll
+      for (int w = 0; w < N; ++w) {
+        float h[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const float keep = b4 ? acc[w][q + 3] : acc[w][q], send = b4 ? acc[w][q] : acc[w][q + 3];
+          h[q] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+        }
+        const float g0 = __shfl_xor_sync(0xffffffffu, b3 ? h[0] : h[2], 8);
+        const float g1 = __shfl_xor_sync(0xffffffffu, h[1], 8);
+        float u = b3 ? h[2] + g0 : h[0] + g0, v = h[1] + g1;  // v: rows 1 and 4, where b3 is 0
+#pragma unroll
+        for (int off = 4; off > 0; off >>= 1) {
+          u += __shfl_xor_sync(0xffffffffu, u, off);
+          v += __shfl_xor_sync(0xffffffffu, v, off);
+        }
+        const float qu = __shfl_sync(0xffffffffu, u, src), qv = __shfl_sync(0xffffffffu, v, src);
+        if (sub == (uint32_t)w) qa = part == 1u ? qv : qu;
+      }
+      if (!own) qa = 0.0f;
       push(s_pq, (double)po * (double)qa);
       team_barrier<C>();
-      const double pq = sum(s_pq);
+      const double pq = totals(s_pq, nullptr).x;
       if (!(pq > 0.0) || !isfinite(pq)) {
         status = 2;  // non-positive curvature: x unchanged
         break;
@@ -256,20 +286,18 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
       precondition();
       publish();
       team_barrier<C>();
-      const double rz_new = sum(s_rz);
-      rr = sum(s_rr);
+      const double2 now = totals(s_rz, s_rr);
+      const double rz_new = now.x;
+      rr = now.y;
       ++iters;
-      if (rr <= stop2 || !(rz_new > 0.0)) {
-        rz = rz_new;
-        break;
-      }
+      const double rz_inv = inv_rz;
+      rz = rz_new;
+      if (rr <= stop2 || !(rz_new > 0.0)) break;
       if (iters >= cap) {
         status = 1;
-        rz = rz_new;
         break;
       }
-      beta = (float)(rz_new * inv_rz);
-      rz = rz_new;
+      beta = (float)(rz_new * rz_inv);
     }
   }
   if (own) d.x[at] = x;
@@ -284,10 +312,10 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
   }
 }
 
-template <int C, int W, int CPL>
+template <int C, int W, int CPL, int N>
 cudaError_t launch_class(const Dev& d, uint32_t begin, uint32_t end, cudaStream_t s) {
   if (begin == end) return cudaSuccess;
-  auto kernel = k_pcg_small<C, W, CPL>;
+  auto kernel = k_pcg_small<C, W, CPL, N>;
   if (C > 8) {  // beyond the portable cluster size
     const cudaError_t e =
         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -318,10 +346,10 @@ int small_pcg_class(uint32_t rows) {
 }
 
 cudaError_t launch_pcg_small(const Dev& d, cudaStream_t s) {
-  cudaError_t e = launch_class<1, 16, 3>(d, d.small_off[0], d.small_off[1], s);
-  if (e == cudaSuccess) e = launch_class<2, 16, 6>(d, d.small_off[1], d.small_off[2], s);
-  if (e == cudaSuccess) e = launch_class<4, 16, 12>(d, d.small_off[2], d.small_off[3], s);
-  if (e == cudaSuccess) e = launch_class<16, 8, 24>(d, d.small_off[3], d.small_off[4], s);
+  cudaError_t e = launch_class<1, 16, 3, 1>(d, d.small_off[0], d.small_off[1], s);
+  if (e == cudaSuccess) e = launch_class<1, 16, 6, 2>(d, d.small_off[1], d.small_off[2], s);
+  if (e == cudaSuccess) e = launch_class<4, 16, 12, 1>(d, d.small_off[2], d.small_off[3], s);
+  if (e == cudaSuccess) e = launch_class<16, 8, 24, 1>(d, d.small_off[3], d.small_off[4], s);
   return e;
 }
 
