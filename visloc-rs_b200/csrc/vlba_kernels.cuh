@@ -144,7 +144,9 @@ struct ElimDev {
 // The pair index: write = false counts each edge's pairs into cursor (zeroed
 // first); write = true writes them at cursor (set to the edges' offsets).
 cudaError_t launch_el_index(const ElimDev& e, bool write, cudaStream_t s);
-cudaError_t launch_el_prepare(const ElimDev& e, cudaStream_t s);
+// The FP32 products with this call's point inverses, and with `hcp` the FP32
+// copies of a new linearisation's blocks.
+cudaError_t launch_el_prepare(const ElimDev& e, bool hcp, cudaStream_t s);
 cudaError_t launch_el_blocks(const ElimDev& e, cudaStream_t s);
 cudaError_t launch_el_outputs(const ElimDev& e, cudaStream_t s);
 

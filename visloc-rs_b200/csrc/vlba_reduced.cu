@@ -490,12 +490,15 @@ __global__ void __launch_bounds__(256) k_el_index(ElimDev E) {
   }
 }
 
-// Per camera-point block o of point p: an FP32 copy of hcp and sk = hcp V_p^-1
-// (formed in FP64; zero for a point left out, whose pairs then add zero).
+// Per camera-point block o of point p: sk = hcp V_p^-1 (formed in FP64; zero for
+// a point left out, whose pairs then add zero), and with HCP, on a new
+// linearisation, an FP32 copy of hcp (the same for every trial of it).
 // One thread per entry q = 6 i + r of the 6x3 outputs, so that consecutive
 // threads read and write consecutive addresses (the three hcp entries an
 // output needs come from the same 144-byte block, through L1).  The FP32
-// copies are kElRec floats apart (80 bytes: five 16-byte loads a block).
+// copies are kElRec floats apart (80 bytes: five 16-byte loads a block; 96
+// bytes read by 32-byte loads took 880 us where these take 760).
+template <bool HCP>
 __global__ void k_el_prepare(ElimDev E) {
   const uint64_t n = 18 * E.num_obs;
   for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n;
@@ -508,7 +511,7 @@ __global__ void k_el_prepare(ElimDev E) {
     const bool used = !E.used || E.used[p];
     const double sk = h[r] * v[3 * i] + h[6 + r] * v[3 * i + 1] + h[12 + r] * v[3 * i + 2];
     E.sk32[kElRec * o + q] = used ? (float)sk : 0.0f;
-    E.hcp32[kElRec * o + q] = (float)h[q];
+    if (HCP) E.hcp32[kElRec * o + q] = (float)h[q];
   }
 }
 
@@ -584,23 +587,26 @@ __global__ void k_el_gather(ElimDev E) {
 }
 
 // coarse_out[g m + h] (g <= h): the sum of the blocks of edges (a, b), a in
-// aggregate g, b in aggregate h, both below coarse_nodes, in node then edge
-// order.  One warp per aggregate pair (g, h), g <= h, lanes over the 36
-// entries.
-__global__ void __launch_bounds__(256) k_el_coarse(ElimDev E) {
+// aggregate g, b in aggregate h, both below coarse_nodes.  One block of
+// kCoarseWarps warps per aggregate pair (g, h), g <= h, lanes over the 36
+// entries: warp w adds the edges of nodes a = w, w + kCoarseWarps, ... of the
+// aggregate in node then edge order, and the warps' sums are added in order
+// (one warp alone walked up to a thousand edges, a chain of loads: 555 us for
+// 29 aggregates of 32 nodes on B200, 26 us with sixteen).
+constexpr int kCoarseWarps = 16;
+__global__ void __launch_bounds__(32 * kCoarseWarps) k_el_coarse(ElimDev E) {
+  __shared__ double part[kCoarseWarps][36];
   const uint32_t m = E.coarse_m, grp = E.coarse_group;
-  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const bool two = lane < 4u;
   const uint64_t npairs = (uint64_t)m * m;
-  const uint64_t nw = (uint64_t)gridDim.x * blockDim.x / 32u;
-  for (uint64_t gh = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32u; gh < npairs;
-       gh += nw) {
+  for (uint64_t gh = blockIdx.x; gh < npairs; gh += gridDim.x) {
     const uint32_t g = (uint32_t)(gh / m), h = (uint32_t)(gh % m);
-    if (h < g) continue;
+    if (h < g) continue;  // the same for the whole block
     const uint32_t a1 = min((g + 1) * grp, E.coarse_nodes);
     const uint32_t t0 = h * grp, t1 = min((h + 1) * grp, E.coarse_nodes);
     double acc0 = 0.0, acc1 = 0.0;
-    for (uint32_t a = g * grp; a < a1; ++a) {
+    for (uint32_t a = g * grp + warp; a < a1; a += kCoarseWarps) {
       uint32_t lo = E.row_off[a], hi = E.row_off[a + 1];
       const uint32_t end = hi;
       while (lo < hi) {
@@ -608,14 +614,28 @@ __global__ void __launch_bounds__(256) k_el_coarse(ElimDev E) {
         if (E.edge_t[mid] < t0) lo = mid + 1;
         else hi = mid;
       }
-      for (uint32_t e = lo; e < end && E.edge_t[e] < t1; ++e) {
+      uint32_t last = lo;
+      for (hi = end; last < hi;) {
+        const uint32_t mid = (last + hi) / 2;
+        if (E.edge_t[mid] < t1) last = mid + 1;
+        else hi = mid;
+      }
+#pragma unroll 4
+      for (uint32_t e = lo; e < last; ++e) {
         acc0 += E.blocks[36 * (size_t)e + lane];
         if (two) acc1 += E.blocks[36 * (size_t)e + 32 + lane];
       }
     }
-    double* out = E.coarse_out + 36 * gh;
-    out[lane] = acc0;
-    if (two) out[32 + lane] = acc1;
+    part[warp][lane] = acc0;
+    if (two) part[warp][32 + lane] = acc1;
+    __syncthreads();
+    if (threadIdx.x < 36) {
+      double t = 0.0;
+#pragma unroll
+      for (int w = 0; w < kCoarseWarps; ++w) t += part[w][threadIdx.x];
+      E.coarse_out[36 * gh + threadIdx.x] = t;
+    }
+    __syncthreads();
   }
 }
 
@@ -671,8 +691,10 @@ cudaError_t launch_el_index(const ElimDev& e, bool write, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_el_prepare(const ElimDev& e, cudaStream_t s) {
-  if (e.num_obs) k_el_prepare<<<flat_grid(18 * e.num_obs), 256, 0, s>>>(e);
+cudaError_t launch_el_prepare(const ElimDev& e, bool hcp, cudaStream_t s) {
+  if (e.num_obs == 0) return cudaSuccess;
+  if (hcp) k_el_prepare<true><<<flat_grid(18 * e.num_obs), 256, 0, s>>>(e);
+  else k_el_prepare<false><<<flat_grid(18 * e.num_obs), 256, 0, s>>>(e);
   return cudaGetLastError();
 }
 
@@ -685,8 +707,8 @@ cudaError_t launch_el_blocks(const ElimDev& e, cudaStream_t s) {
 cudaError_t launch_el_outputs(const ElimDev& e, cudaStream_t s) {
   if (e.num_run) k_el_gather<<<flat_grid(36 * e.num_run), 256, 0, s>>>(e);
   if (e.coarse_m)
-    k_el_coarse<<<(int)std::min<uint64_t>(((uint64_t)e.coarse_m * e.coarse_m + 7) / 8, 148 * 16),
-                  256, 0, s>>>(e);
+    k_el_coarse<<<(int)std::min<uint64_t>((uint64_t)e.coarse_m * e.coarse_m, 148 * 16),
+                  32 * kCoarseWarps, 0, s>>>(e);
   return cudaGetLastError();
 }
 

@@ -2657,12 +2657,12 @@ bool reduced_eliminate(Context* c, const vlba_point_elimination* el, double* run
     E.num_obs = nobs;
     E.structure_id = el->structure_id;
   }
-  if (!E.hcp_valid || E.linearization_id != el->linearization_id) {
+  const bool new_hcp = !E.hcp_valid || E.linearization_id != el->linearization_id;
+  if (new_hcp) {
+    E.hcp_valid = false;
     Stager st(c);
     st.add(E.hcp64.p, el->hcp, 144 * nobs);
     st.flush(s);
-    E.hcp_valid = true;
-    E.linearization_id = el->linearization_id;
   }
   // Per call: the point inverses, the couplings (merged per edge in their
   // order), the run edges and the outputs.
@@ -2732,7 +2732,9 @@ bool reduced_eliminate(Context* c, const vlba_point_elimination* el, double* run
   d.run_edges = E.run_edges.as<const uint32_t>();
   d.run_out = E.run_out.as<double>();
   d.coarse_out = E.coarse_out.as<double>();
-  check_launch(launch_el_prepare(d, s), "elimination prepare");
+  check_launch(launch_el_prepare(d, new_hcp, s), "elimination prepare");
+  E.hcp_valid = true;
+  E.linearization_id = el->linearization_id;
   check_launch(launch_el_blocks(d, s), "elimination blocks");
   check_launch(launch_el_outputs(d, s), "elimination outputs");
   VLBA_CUDA(cudaEventRecord(c->ev[5], s));
