@@ -17,7 +17,9 @@
 //                   reduced rhs and the FP64 6x6 Cholesky block-Jacobi inverse
 //                                                      (ba.wgsl:141-183, 263-387)
 //   k_pcg           persistent: block-Jacobi PCG on S, tiles of S streamed
-//                   HBM -> shared memory by TMA bulk copies (ba.wgsl:420-562)
+//                   HBM -> shared memory by TMA bulk copies (ba.wgsl:420-562);
+//                   systems that fit the chip go to k_pcg_small and k_pcg_team
+//                   (vlba_pcg_small.cu, vlba_pcg_team.cu)
 //   k_pose_update   T <- T Exp(xi) in FP64             (solver.rs:599-607)
 //   k_cost<true>    back-substitution dl = -H^-1 (g + sum W^T dc), then the
 //                   FP64 robust cost and non-projectable count of the trial
@@ -127,39 +129,6 @@ __device__ __forceinline__ void reduce_cost(double& cost, unsigned long long& ba
     }
   }
   __syncthreads();
-}
-
-// 6x6 SPD inverse by Cholesky in FP64; false if not positive definite.
-__device__ bool chol_inverse6(const double* a, double* inv) {
-  double L[36];
-#pragma unroll
-  for (int e = 0; e < 36; ++e) L[e] = a[e];
-  for (int j = 0; j < 6; ++j) {
-    double s = L[j * 6 + j];
-    for (int q = 0; q < j; ++q) s -= L[j * 6 + q] * L[j * 6 + q];
-    if (!(s > 0.0) || !isfinite(s)) return false;
-    const double ljj = sqrt(s);
-    L[j * 6 + j] = ljj;
-    for (int i = j + 1; i < 6; ++i) {
-      double t = L[i * 6 + j];
-      for (int q = 0; q < j; ++q) t -= L[i * 6 + q] * L[j * 6 + q];
-      L[i * 6 + j] = t / ljj;
-    }
-  }
-  for (int c = 0; c < 6; ++c) {
-    double y[6];
-    for (int i = 0; i < 6; ++i) {
-      double s = (i == c) ? 1.0 : 0.0;
-      for (int q = 0; q < i; ++q) s -= L[i * 6 + q] * y[q];
-      y[i] = s / L[i * 6 + i];
-    }
-    for (int ii = 5; ii >= 0; --ii) {
-      double s = y[ii];
-      for (int q = ii + 1; q < 6; ++q) s -= L[q * 6 + ii] * inv[q * 6 + c];
-      inv[ii * 6 + c] = s / L[ii * 6 + ii];
-    }
-  }
-  return true;
 }
 
 // 32-byte vector load (read-only path) and store: one request per 32-byte
@@ -2210,41 +2179,48 @@ __global__ void __launch_bounds__(Pcg::kThreads, 1) k_pcg(Dev d) {
 // tile); node i's damped diagonal block, column-major
 // f64, to its diagonal slot, its FP64 Cholesky inverse (the block-Jacobi
 // preconditioner; the diagonal's inverse if not positive definite) and its
-// rhs.  Padding slots keep zero blocks, preconditioner and rhs.
+// rhs.  Padding slots keep zero blocks, preconditioner and rhs.  One thread
+// per entry of an off-diagonal block, so that a warp reads and writes
+// consecutive addresses, and a warp per node (a thread per block and per node
+// took 77 us for 202,000 blocks of 1,500 nodes on B200, this 44).
 __global__ void __launch_bounds__(256) k_reduced_fill(Dev d, uint32_t n, uint64_t ne,
                                                       const double* diag, const float* offdiag,
                                                       const double* offdiag64,
                                                       const double* rhs) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < ne; e += stride) {
+  const uint64_t first = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  for (uint64_t j = first; j < 36 * ne; j += stride) {
+    const uint64_t e = j / 36;
+    const uint32_t q = (uint32_t)(j - 36 * e), r = q % 6, c = q / 6;
     const uint2 dst = d.blk_dst[e];
+    const float v = offdiag ? offdiag[j] : (float)offdiag64[j];
+    d.tiles[dst.x + r * 6 + c] = v;
+    if (dst.y != kNone) d.tiles[dst.y + c * 6 + r] = v;
+  }
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint64_t i = first / 32; i < d.num_var_cams; i += stride / 32) {
+    if (i >= n) {
+      for (uint32_t e = lane; e < 36; e += 32) d.minv[36 * i + e] = 0.0f;
+      if (lane < 6) d.rhs[6 * i + lane] = 0.0f;
+      continue;
+    }
+    const double* a = diag + 36 * i;
+    double u[21], col[6];
 #pragma unroll
     for (int r = 0; r < 6; ++r)
 #pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        const float v = offdiag ? offdiag[36 * e + c * 6 + r] : (float)offdiag64[36 * e + c * 6 + r];
-        d.tiles[dst.x + r * 6 + c] = v;
-        if (dst.y != kNone) d.tiles[dst.y + c * 6 + r] = v;
+      for (int c = r; c < 6; ++c) u[ut6(r, c)] = a[6 * r + c];  // entry (c, r)
+    float* blk = d.tiles + d.diag_dst[i];
+    for (uint32_t e = lane; e < 36; e += 32) blk[e] = (float)a[e % 6 * 6 + e / 6];
+    const bool ok = chol_column6(u, lane, col);
+    if (lane < 6) {
+#pragma unroll
+      for (int r = 0; r < 6; ++r) {
+        const double fallback = r == (int)lane ? 1.0 / fmax(a[7 * lane], 1e-20) : 0.0;
+        d.minv[36 * i + r * 6 + lane] = (float)(ok ? col[r] : fallback);
       }
-  }
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < d.num_var_cams;
-       i += stride) {
-    double a[36], inv[36];
-    if (i < n) {
-      for (int r = 0; r < 6; ++r)
-        for (int c = 0; c < 6; ++c) a[r * 6 + c] = diag[36 * i + c * 6 + r];
-      float* blk = d.tiles + d.diag_dst[i];
-      for (int e2 = 0; e2 < 36; ++e2) blk[e2] = (float)a[e2];
-      if (!chol_inverse6(a, inv)) {
-        for (int e2 = 0; e2 < 36; ++e2) inv[e2] = 0.0;
-        for (int q = 0; q < 6; ++q) inv[q * 7] = 1.0 / fmax(a[q * 7], 1e-20);
-      }
-      for (int q = 0; q < 6; ++q) d.rhs[6 * i + q] = (float)rhs[6 * i + q];
-    } else {
-      for (int e2 = 0; e2 < 36; ++e2) inv[e2] = 0.0;
-      for (int q = 0; q < 6; ++q) d.rhs[6 * i + q] = 0.0f;
+      d.rhs[6 * i + lane] = (float)rhs[6 * i + lane];
     }
-    for (int e2 = 0; e2 < 36; ++e2) d.minv[36 * i + e2] = (float)inv[e2];
   }
 }
 
@@ -2446,7 +2422,7 @@ int pcg_rows_per_block() { return Pcg::kOwnMax; }
 cudaError_t launch_reduced_fill(const Dev& d, uint32_t n, uint64_t ne, const double* diag,
                                 const float* offdiag, const double* offdiag64, const double* rhs,
                                 cudaStream_t s) {
-  const size_t work = std::max<size_t>((size_t)ne, d.num_var_cams);
+  const size_t work = std::max<size_t>(36 * (size_t)ne, 32 * (size_t)d.num_var_cams);
   k_reduced_fill<<<grid1d(work, 256), 256, 0, s>>>(d, n, ne, diag, offdiag, offdiag64, rhs);
   return cudaGetLastError();
 }
