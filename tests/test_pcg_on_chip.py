@@ -106,6 +106,20 @@ def test_stopping_rules(solver, n):
     assert it == 0 and not x.any()
 
 
+@pytest.mark.parametrize("cameras", [12, 40, 60, 100, 150, 620])
+def test_a_negative_tolerance_is_never_met(solver, cameras):
+    """|r| <= tol |b| cannot hold for tol < 0: every kernel runs to the cap
+    (with the square of the bound it held once |r| <= |b|)."""
+    p = synth.ring_problem(cameras, 40 * cameras, seed=cameras)
+    cfg = BaConfig(robust_kernel=RobustKernel.huber(1.0), max_pcg_iterations=9)
+    cfg.pcg_relative_tolerance = -1.0
+    never = solver.linear_step(p, cfg, 1e-3)
+    assert never[2] == 9
+    cfg.pcg_relative_tolerance = 0.0
+    zero = solver.linear_step(p, cfg, 1e-3)
+    assert zero[2] == 9 and np.array_equal(never[0], zero[0])
+
+
 @pytest.mark.parametrize("band", [2, 9, 40])
 def test_banded_team(solver, band):
     """A long chain (1,400 nodes, more tile rows than blocks at the widest

@@ -224,7 +224,8 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
   double rz = first.x, rr = first.y;
   const LmParams& lp = d.params[P];
   const double bnorm = sqrt(rr);
-  const double stop = lp.pcg_relative_tolerance * bnorm, stop2 = stop * stop;
+  // |r| <= stop without the root: on squares; a negative tolerance is never met.
+  const double stop = lp.pcg_relative_tolerance * bnorm, stop2 = stop >= 0.0 ? stop * stop : -1.0;
   const uint32_t cap = lp.max_pcg_iterations;
   uint32_t iters = 0, status = 0;
   // pcg_init (ba.wgsl:420-439): done when |b| = 0 or r.z <= 0.

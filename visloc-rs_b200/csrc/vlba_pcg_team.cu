@@ -313,8 +313,9 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pcg_team(Dev d) {
     exchange_z();
     double rz = total(s_rz), rr = total(s_rr);
     const LmParams& lp = d.params[P];
-    const double bnorm = sqrt(rr), stop = lp.pcg_relative_tolerance * bnorm,
-                 stop2 = stop * stop;
+    const double bnorm = sqrt(rr), stop = lp.pcg_relative_tolerance * bnorm;
+    // |r| <= stop without the root: on squares; a negative tolerance is never met.
+    const double stop2 = stop >= 0.0 ? stop * stop : -1.0;
     const uint32_t cap = lp.max_pcg_iterations;
     uint32_t iters = 0, status = 0;
     // pcg_init (ba.wgsl:420-439): done when |b| = 0 or r.z <= 0.
