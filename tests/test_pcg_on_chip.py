@@ -164,3 +164,16 @@ def test_teams_solve_the_same_alone_and_in_a_batch(solver):
         for a, b, c, r in zip(alone, batch, costs, results):
             assert r.final_cost == c
             assert np.array_equal(a.pose_q, b.pose_q) and np.array_equal(a.landmarks, b.landmarks)
+
+
+def test_each_round_of_teams_is_a_launch(solver):
+    """A team's waits never cover another team's solve: two teams that do not
+    fit the device together (112 blocks each) take a launch each."""
+    one = synth.ring_problem(300, 20000, seed=4)
+    cfg = BaConfig(max_iterations=2, robust_kernel=RobustKernel.huber(1.0), max_pcg_iterations=20)
+    st, alone = solver.optimize(one.copy(), cfg)
+    assert st == 0
+    statuses, both = solver.batch_optimize([one.copy(), one.copy()], cfg)
+    assert statuses == [0, 0]
+    assert both[0].kernel_launches == alone.kernel_launches + 2
+    assert both[0].final_cost == both[1].final_cost == alone.final_cost

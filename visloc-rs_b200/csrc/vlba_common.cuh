@@ -169,11 +169,11 @@ struct Dev {
   const uint32_t* small_list;
   uint32_t small_off[kSmallPcgClasses + 1];
   uint32_t num_big;
-  // The problems solved by teams of blocks: team_rounds rounds of team_grid
-  // blocks, each entry of team_sched a block of team_cta or kNone.
-  uint32_t team_rounds, team_grid, team_smem, team_slots_total;
+  // The problems solved by teams of blocks, a launch per round: round r runs
+  // the blocks [team_round_begin[r], team_round_begin[r + 1]) of team_cta.
+  uint32_t team_rounds, team_smem, team_slots_total;
+  const uint32_t* team_round_begin;  // host memory, the context's
   const TeamCta* team_cta;
-  const uint32_t* team_sched;
   const uint32_t* team_cols;
   const uint32_t* team_ents;
   unsigned long long* team_z;      // (exchange number, z), each block's on lines of its own

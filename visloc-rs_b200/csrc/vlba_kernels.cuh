@@ -34,12 +34,12 @@ cudaError_t launch_pcg_small(const Dev& d, cudaStream_t s);
 int small_pcg_class(uint32_t rows);
 
 // The problems past the small classes whose S fits the shared memory of a team
-// of blocks (vlba_pcg_team.cu): the teams' blocks and their rounds.
+// of blocks (vlba_pcg_team.cu): the teams' blocks, and the rounds of teams that
+// fit the device together (round r: blocks round_begin[r] to round_begin[r + 1]).
 struct TeamPlan {
   std::vector<TeamCta> cta;
-  std::vector<uint32_t> sched, cols, ents;
+  std::vector<uint32_t> round_begin, cols, ents;
   std::vector<uint8_t> in_team;  // [num_problems]
-  uint32_t rounds = 0, grid = 0;
   size_t smem = 0;  // the largest block's dynamic shared memory
   uint64_t z_words = 0;
 };

@@ -126,339 +126,331 @@ __device__ __forceinline__ bool gather_slots(const unsigned long long* slots, ui
   return ok;
 }
 
-__global__ void __launch_bounds__(kTeamThreads, 1) k_pcg_team(Dev d) {
+__global__ void __launch_bounds__(kTeamThreads, 1) k_pcg_team(Dev d, uint32_t first) {
   extern __shared__ __align__(16) float smem[];
   __shared__ double s_a[kTeamWarps], s_b[kTeamWarps], s_rz[kTeamPolls], s_rr[kTeamPolls],
       s_pq[kTeamPolls];
   __shared__ int s_fail;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   if (tid == 0) s_fail = 0;
-  for (uint32_t round = 0; round < d.team_rounds; ++round) {
-    const uint32_t idx = d.team_sched[round * d.team_grid + blockIdx.x];
-    if (idx == kNone) continue;
-    const TeamCta T = d.team_cta[idx];
-    const uint32_t P = T.prob;
-    if (d.ctrl[P].done) continue;  // the same for the whole team
-    const uint32_t nn = T.node1 - T.node0, L = 48u * T.ncols, nseg = (T.ncols + kSegTiles - 1) / kSegTiles;
-    const uint32_t parts = nn * nseg, Lp = nseg * kSegment;
-    const uint32_t tr0 = d.prob_tr_begin[P], slot0 = 8u * tr0;
-    const uint32_t* cols = d.team_cols + T.col_begin;  // tile rows (of the problem), ascending
-    const uint32_t staged = max(min(parts, kRegParts), parts > kRegParts ? parts - kRegParts : 0u);
-    float* const S = smem;                                  // [staged] parts of [6][kSegment]
-    float* const p = S + (size_t)staged * kPartFloats;      // [Lp], zero past L
-    float* const z_in = p + Lp;                             // [L]
-    float* const part = z_in + Lp;                          // [nseg][6 nn] products
-    // Where each pair of the block's columns finds its z.
-    uint32_t* const z_at = reinterpret_cast<uint32_t*>(part + (size_t)nseg * 6 * nn);  // [L / 2]
-    const unsigned long long* const zw = d.team_z + T.z_team;
-    unsigned long long* const z_mine = d.team_z + T.z_team + T.z_own;
-    unsigned long long* const pq_slots = d.team_slots + kLineWords * (size_t)T.slot_base;
-    unsigned long long* const rz_slots = pq_slots + kLineWords * (size_t)d.team_slots_total;
-    __syncthreads();  // shared memory of the round before is free
+  const TeamCta T = d.team_cta[first + blockIdx.x];
+  const uint32_t P = T.prob;
+  if (d.ctrl[P].done) return;  // the same for the whole team
+  const uint32_t nn = T.node1 - T.node0, L = 48u * T.ncols, nseg = (T.ncols + kSegTiles - 1) / kSegTiles;
+  const uint32_t parts = nn * nseg, Lp = nseg * kSegment;
+  const uint32_t tr0 = d.prob_tr_begin[P], slot0 = 8u * tr0;
+  const uint32_t* cols = d.team_cols + T.col_begin;  // tile rows (of the problem), ascending
+  const uint32_t staged = max(min(parts, kRegParts), parts > kRegParts ? parts - kRegParts : 0u);
+  float* const S = smem;                                  // [staged] parts of [6][kSegment]
+  float* const p = S + (size_t)staged * kPartFloats;      // [Lp], zero past L
+  float* const z_in = p + Lp;                             // [L]
+  float* const part = z_in + Lp;                          // [nseg][6 nn] products
+  // Where each pair of the block's columns finds its z.
+  uint32_t* const z_at = reinterpret_cast<uint32_t*>(part + (size_t)nseg * 6 * nn);  // [L / 2]
+  const unsigned long long* const zw = d.team_z + T.z_team;
+  unsigned long long* const z_mine = d.team_z + T.z_team + T.z_own;
+  unsigned long long* const pq_slots = d.team_slots + kLineWords * (size_t)T.slot_base;
+  unsigned long long* const rz_slots = pq_slots + kLineWords * (size_t)d.team_slots_total;
 
-    // Part q (camera q % nn, segment q / nn) of the block's rows of S: parts
-    // [q0, q1) into shared memory, a camera and tile column per warp at a time.
-    auto stage = [&](uint32_t q0, uint32_t q1) {
-      for (uint32_t it = warp; it < (q1 - q0) * kSegTiles; it += kTeamWarps) {
-        const uint32_t q = q0 + it / kSegTiles, kk = it % kSegTiles;
-        const uint32_t node = T.node0 + q % nn, k = q / nn * kSegTiles + kk;
-        const uint32_t I = node >> 3, li = node & 7u, J = k < T.ncols ? cols[k] : 0u;
-        const uint32_t t = k < T.ncols ? d.team_ents[T.ent_begin + (I - (T.node0 >> 3)) * T.ncols + k]
-                                       : kNone;
-        float* dst = S + (size_t)(q - q0) * kPartFloats + 48u * kk;
-        const float* src = d.tiles + (size_t)t * (64 * kBlock) + (I >= J ? li * 288u : li * 36u);
+  // Part q (camera q % nn, segment q / nn) of the block's rows of S: parts
+  // [q0, q1) into shared memory, a camera and tile column per warp at a time.
+  auto stage = [&](uint32_t q0, uint32_t q1) {
+    for (uint32_t it = warp; it < (q1 - q0) * kSegTiles; it += kTeamWarps) {
+      const uint32_t q = q0 + it / kSegTiles, kk = it % kSegTiles;
+      const uint32_t node = T.node0 + q % nn, k = q / nn * kSegTiles + kk;
+      const uint32_t I = node >> 3, li = node & 7u, J = k < T.ncols ? cols[k] : 0u;
+      const uint32_t t = k < T.ncols ? d.team_ents[T.ent_begin + (I - (T.node0 >> 3)) * T.ncols + k]
+                                     : kNone;
+      float* dst = S + (size_t)(q - q0) * kPartFloats + 48u * kk;
+      const float* src = d.tiles + (size_t)t * (64 * kBlock) + (I >= J ? li * 288u : li * 36u);
 #pragma unroll
-        for (int i = 0; i < 9; ++i) {
-          const uint32_t e = lane + 32u * i, lj = e / 36u, w = e % 36u;
-          // Below or on the diagonal: block (li, lj) row by row; above it: the
-          // mirrored block (lj, li) column by column.
-          const float v = t == kNone ? 0.0f : (I >= J ? src[e] : src[lj * 288u + w]);
-          const uint32_t a = I >= J ? w / 6u : w % 6u, c = I >= J ? w % 6u : w / 6u;
-          dst[a * kSegment + lj * 6u + c] = v;
+      for (int i = 0; i < 9; ++i) {
+        const uint32_t e = lane + 32u * i, lj = e / 36u, w = e % 36u;
+        // Below or on the diagonal: block (li, lj) row by row; above it: the
+        // mirrored block (lj, li) column by column.
+        const float v = t == kNone ? 0.0f : (I >= J ? src[e] : src[lj * 288u + w]);
+        const uint32_t a = I >= J ? w / 6u : w % 6u, c = I >= J ? w % 6u : w / 6u;
+        dst[a * kSegment + lj * 6u + c] = v;
+      }
+    }
+  };
+  float4 Sr[kHeld][6][kSegVec];  // this warp's parts: warp, warp + kTeamWarps
+  stage(0, min(parts, kRegParts));
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u) {
+    const uint32_t it = warp + u * kTeamWarps;
+    const float4* s4 = reinterpret_cast<const float4*>(S + (size_t)it * kPartFloats);
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
+#pragma unroll
+      for (int j = 0; j < kSegVec; ++j)
+        Sr[u][q][j] = it < parts ? s4[q * (kSegment / 4) + lane + 32 * j]
+                                 : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  }
+  if (parts > kRegParts) {
+    __syncthreads();
+    stage(kRegParts, parts);
+  }
+  uint32_t node_held[kHeld], seg_held[kHeld];
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u) {
+    const uint32_t it = min(warp + u * kTeamWarps, parts - 1u);
+    node_held[u] = it % nn;
+    seg_held[u] = it / nn;
+  }
+  for (uint32_t e = tid; e < Lp; e += kTeamThreads) p[e] = 0.0f;
+  for (uint32_t e = 2u * tid; e < L; e += 2u * kTeamThreads) {
+    // The owner of a camera: the last block whose first camera is not past it.
+    const uint32_t entry = 48u * cols[e / 48u] + e % 48u, node = entry / 6u;
+    uint32_t g = (uint32_t)((uint64_t)node * T.size / (8u * (d.prob_tr_begin[P + 1] - tr0)));
+    const TeamCta* team = d.team_cta + T.slot_base;
+    while (g + 1 < T.size && team[g + 1].node0 <= node) ++g;
+    while (team[g].node0 > node) --g;
+    z_at[e / 2u] = team[g].z_own + entry - 6u * team[g].node0;
+  }
+
+  // Eight threads a camera: vector entry a of camera gi.
+  const uint32_t gi = tid >> 3, a = tid & 7u;
+  const bool own = gi < nn && a < 6u;
+  const uint32_t nwarp = (nn + 3) / 4;  // warps that own cameras
+  const size_t at = (size_t)6 * (slot0 + T.node0 + gi) + a;
+  float m[6];
+#pragma unroll
+  for (int b = 0; b < 6; ++b) m[b] = own ? d.minv[6 * at + b] : 0.0f;
+  float x = 0.0f, r = own ? d.rhs[at] : 0.0f, z = 0.0f, po = 0.0f;
+  const uint32_t epoch0 = d.team_epoch[P];
+  uint32_t epoch = epoch0;
+
+  // The team's total from the polling warps' sums, in order.
+  auto total = [&](const double* s) {
+    double v = 0.0;
+#pragma unroll
+    for (int i = 0; i < kTeamPolls; ++i) v += 32u * i < T.size ? s[i] : 0.0;
+    return v;
+  };
+  bool ok = true;
+  // z = M^-1 r, published with the block's r.z and r.r; waits for the
+  // team's slots (their sums in s_rz and s_rr) and the z of the block's
+  // columns.
+  auto exchange_z = [&]() {
+    ++epoch;
+    z = 0.0f;
+#pragma unroll
+    for (int b = 0; b < 6; ++b) z += m[b] * __shfl_sync(0xffffffffu, r, b, 8);
+    if (own) put_word(z_mine + 6 * gi + a, __float_as_uint(z), epoch);
+    double rz = 0.0, rr = 0.0;
+    if (warp < nwarp) {
+      rz = warp_sum_t((double)r * (double)z);
+      rr = warp_sum_t((double)r * (double)r);
+      if (lane == 0) {
+        s_a[warp] = rz;
+        s_b[warp] = rr;
+      }
+    }
+    if (nwarp > 1) __syncthreads();
+    if (warp == 0) {
+      for (uint32_t w = 1; w < nwarp; ++w) {
+        rz += s_a[w];
+        rr += s_b[w];
+      }
+      if (lane < 4u) {
+        const double s = lane < 2u ? rz : rr;
+        put_word(rz_slots + kLineWords * T.rank + lane,
+                 (uint32_t)((lane & 1u) ? __double2hiint(s) : __double2loint(s)), epoch);
+      }
+    }
+    if (32u * warp < T.size) {
+      double sum[2];
+      const bool got = gather_slots<2>(rz_slots, T.size, epoch, sum);
+      if (lane == 0) {
+        s_rz[warp] = sum[0];
+        s_rr[warp] = sum[1];
+        if (!got) s_fail = 1;
+      }
+    }
+    __syncthreads();
+    // A wait that gives up has lasted kWaitLimitNs: no thread sets s_fail
+    // while another is still on its way here.  One that gives up below is
+    // seen at the next check.
+    ok = s_fail == 0;
+    if (!ok) return;
+    // The team's z is there or about to be (each block stored it before its
+    // slot): read only now, so that early polls do not crowd the stores.
+    for (uint32_t e0 = 2u * tid; e0 < L; e0 += 2u * kInFlight * kTeamThreads) {
+      unsigned long long v[kInFlight][2];
+      const unsigned long long* w[kInFlight];
+#pragma unroll
+      for (int i = 0; i < kInFlight; ++i) {
+        const uint32_t e = min(e0 + i * 2u * kTeamThreads, L - 2u);
+        w[i] = zw + z_at[e / 2u];
+        get_words(w[i], v[i][0], v[i][1]);
+      }
+      Deadline dl;
+#pragma unroll
+      for (int i = 0; i < kInFlight; ++i) {
+        while (!fresh(v[i][0], epoch) || !fresh(v[i][1], epoch)) {
+          if (!dl.wait()) {
+            s_fail = 1;
+            break;
+          }
+          get_words(w[i], v[i][0], v[i][1]);
+        }
+        const uint32_t e = e0 + i * 2u * kTeamThreads;
+        if (e < L)
+          *reinterpret_cast<float2*>(z_in + e) =
+              make_float2(__uint_as_float((uint32_t)v[i][0]), __uint_as_float((uint32_t)v[i][1]));
+      }
+    }
+    // Each thread updates the entries of p that it read: the next barrier
+    // is the one before the product.
+  };
+
+  exchange_z();
+  double rz = total(s_rz), rr = total(s_rr);
+  const LmParams& lp = d.params[P];
+  const double bnorm = sqrt(rr), stop = lp.pcg_relative_tolerance * bnorm;
+  // |r| <= stop without the root: on squares; a negative tolerance is never met.
+  const double stop2 = stop >= 0.0 ? stop * stop : -1.0;
+  const uint32_t cap = lp.max_pcg_iterations;
+  uint32_t iters = 0, status = 0;
+  // pcg_init (ba.wgsl:420-439): done when |b| = 0 or r.z <= 0.
+  if (ok && rr > 0.0 && rz > 0.0 && cap != 0u) {
+    float beta = 0.0f;
+    for (;;) {
+      const double inv_rz = inverse64(rz);
+      for (uint32_t e = 2u * tid; e < L; e += 2u * kTeamThreads) {
+        const float2 zv = *reinterpret_cast<const float2*>(z_in + e);
+        float2 pv = *reinterpret_cast<const float2*>(p + e);
+        pv.x = __fmaf_rn(beta, pv.x, zv.x);
+        pv.y = __fmaf_rn(beta, pv.y, zv.y);
+        *reinterpret_cast<float2*>(p + e) = pv;
+      }
+      po = __fmaf_rn(beta, po, z);
+      __syncthreads();
+      // Row sums of a part: the lanes' products by a reduce-scatter over
+      // bits 4 and 3, then a butterfly.
+      auto reduce = [&](const float (&acc)[6], uint32_t node, uint32_t seg, bool store) {
+        const bool b4 = (lane >> 4) & 1u, b3 = (lane >> 3) & 1u;
+        float h[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const float keep = b4 ? acc[q + 3] : acc[q], send = b4 ? acc[q] : acc[q + 3];
+          h[q] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+        }
+        const float g0 = __shfl_xor_sync(0xffffffffu, b3 ? h[0] : h[2], 8);
+        const float g1 = __shfl_xor_sync(0xffffffffu, h[1], 8);
+        float u = b3 ? h[2] + g0 : h[0] + g0, v = h[1] + g1;
+#pragma unroll
+        for (int off = 4; off > 0; off >>= 1) {
+          u += __shfl_xor_sync(0xffffffffu, u, off);
+          v += __shfl_xor_sync(0xffffffffu, v, off);
+        }
+        float* out = part + (size_t)seg * 6 * nn + 6 * node + (b4 ? 3 : 0);
+        if (store && (lane & 7u) == 0) out[b3 ? 2 : 0] = u;
+        if (store && (lane & 15u) == 1) out[1] = v;
+      };
+      auto madd = [](float4 s, float4 v, float& acc) {
+        acc = __fmaf_rn(s.x, v.x, acc);
+        acc = __fmaf_rn(s.y, v.y, acc);
+        acc = __fmaf_rn(s.z, v.z, acc);
+        acc = __fmaf_rn(s.w, v.w, acc);
+      };
+      const float4* p4 = reinterpret_cast<const float4*>(p);
+      // The held parts' products, then their reductions side by side (a
+      // part past the last holds zeros and stores nothing).
+      float held[kHeld][6];
+#pragma unroll
+      for (int u = 0; u < kHeld; ++u) {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) held[u][q] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < kSegVec; ++j) {
+          const float4 pv = p4[seg_held[u] * (kSegment / 4) + lane + 32 * j];
+#pragma unroll
+          for (int q = 0; q < 6; ++q) madd(Sr[u][q][j], pv, held[u][q]);
         }
       }
-    };
-    float4 Sr[kHeld][6][kSegVec];  // this warp's parts: warp, warp + kTeamWarps
-    stage(0, min(parts, kRegParts));
-    __syncthreads();
 #pragma unroll
-    for (int u = 0; u < kHeld; ++u) {
-      const uint32_t it = warp + u * kTeamWarps;
-      const float4* s4 = reinterpret_cast<const float4*>(S + (size_t)it * kPartFloats);
+      for (int u = 0; u < kHeld; ++u)
+        reduce(held[u], node_held[u], seg_held[u], warp + u * kTeamWarps < parts);
+      for (uint32_t it = kRegParts + warp; it < parts; it += kTeamWarps) {
+        const uint32_t node = it % nn, seg = it / nn;
+        const float4* s4 = reinterpret_cast<const float4*>(S + (size_t)(it - kRegParts) * kPartFloats);
+        float acc[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 1
+        for (int j = 0; j < kSegVec; ++j) {
+          const float4 pv = p4[seg * (kSegment / 4) + lane + 32 * j];
 #pragma unroll
-      for (int q = 0; q < 6; ++q)
-#pragma unroll
-        for (int j = 0; j < kSegVec; ++j)
-          Sr[u][q][j] = it < parts ? s4[q * (kSegment / 4) + lane + 32 * j]
-                                   : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
-    if (parts > kRegParts) {
-      __syncthreads();
-      stage(kRegParts, parts);
-    }
-    uint32_t node_held[kHeld], seg_held[kHeld];
-#pragma unroll
-    for (int u = 0; u < kHeld; ++u) {
-      const uint32_t it = min(warp + u * kTeamWarps, parts - 1u);
-      node_held[u] = it % nn;
-      seg_held[u] = it / nn;
-    }
-    for (uint32_t e = tid; e < Lp; e += kTeamThreads) p[e] = 0.0f;
-    for (uint32_t e = 2u * tid; e < L; e += 2u * kTeamThreads) {
-      // The owner of a camera: the last block whose first camera is not past it.
-      const uint32_t entry = 48u * cols[e / 48u] + e % 48u, node = entry / 6u;
-      uint32_t g = (uint32_t)((uint64_t)node * T.size / (8u * (d.prob_tr_begin[P + 1] - tr0)));
-      const TeamCta* team = d.team_cta + T.slot_base;
-      while (g + 1 < T.size && team[g + 1].node0 <= node) ++g;
-      while (team[g].node0 > node) --g;
-      z_at[e / 2u] = team[g].z_own + entry - 6u * team[g].node0;
-    }
-
-    // Eight threads a camera: vector entry a of camera gi.
-    const uint32_t gi = tid >> 3, a = tid & 7u;
-    const bool own = gi < nn && a < 6u;
-    const uint32_t nwarp = (nn + 3) / 4;  // warps that own cameras
-    const size_t at = (size_t)6 * (slot0 + T.node0 + gi) + a;
-    float m[6];
-#pragma unroll
-    for (int b = 0; b < 6; ++b) m[b] = own ? d.minv[6 * at + b] : 0.0f;
-    float x = 0.0f, r = own ? d.rhs[at] : 0.0f, z = 0.0f, po = 0.0f;
-    const uint32_t epoch0 = d.team_epoch[P];
-    uint32_t epoch = epoch0;
-
-    // The team's total from the polling warps' sums, in order.
-    auto total = [&](const double* s) {
-      double v = 0.0;
-#pragma unroll
-      for (int i = 0; i < kTeamPolls; ++i) v += 32u * i < T.size ? s[i] : 0.0;
-      return v;
-    };
-    bool ok = true;
-    // z = M^-1 r, published with the block's r.z and r.r; waits for the
-    // team's slots (their sums in s_rz and s_rr) and the z of the block's
-    // columns.
-    auto exchange_z = [&]() {
-      ++epoch;
-      z = 0.0f;
-#pragma unroll
-      for (int b = 0; b < 6; ++b) z += m[b] * __shfl_sync(0xffffffffu, r, b, 8);
-      if (own) put_word(z_mine + 6 * gi + a, __float_as_uint(z), epoch);
-      double rz = 0.0, rr = 0.0;
-      if (warp < nwarp) {
-        rz = warp_sum_t((double)r * (double)z);
-        rr = warp_sum_t((double)r * (double)r);
-        if (lane == 0) {
-          s_a[warp] = rz;
-          s_b[warp] = rr;
+          for (int q = 0; q < 6; ++q) madd(s4[q * (kSegment / 4) + lane + 32 * j], pv, acc[q]);
         }
+        reduce(acc, node, seg, true);
+      }
+      __syncthreads();
+      float qa = 0.0f;
+      if (own)
+        for (uint32_t s = 0; s < nseg; ++s) qa += part[(size_t)s * 6 * nn + 6 * gi + a];
+      ++epoch;
+      double pq_own = 0.0;
+      if (warp < nwarp) {
+        pq_own = warp_sum_t((double)po * (double)qa);
+        if (lane == 0) s_a[warp] = pq_own;
       }
       if (nwarp > 1) __syncthreads();
       if (warp == 0) {
-        for (uint32_t w = 1; w < nwarp; ++w) {
-          rz += s_a[w];
-          rr += s_b[w];
-        }
-        if (lane < 4u) {
-          const double s = lane < 2u ? rz : rr;
-          put_word(rz_slots + kLineWords * T.rank + lane,
-                   (uint32_t)((lane & 1u) ? __double2hiint(s) : __double2loint(s)), epoch);
-        }
+        for (uint32_t w = 1; w < nwarp; ++w) pq_own += s_a[w];
+        if (lane < 2u)
+          put_word(pq_slots + kLineWords * T.rank + lane,
+                   (uint32_t)(lane ? __double2hiint(pq_own) : __double2loint(pq_own)), epoch);
       }
       if (32u * warp < T.size) {
-        double sum[2];
-        const bool got = gather_slots<2>(rz_slots, T.size, epoch, sum);
+        double sum[1];
+        const bool got = gather_slots<1>(pq_slots, T.size, epoch, sum);
         if (lane == 0) {
-          s_rz[warp] = sum[0];
-          s_rr[warp] = sum[1];
+          s_pq[warp] = sum[0];
           if (!got) s_fail = 1;
         }
       }
       __syncthreads();
-      // A wait that gives up has lasted kWaitLimitNs: no thread sets s_fail
-      // while another is still on its way here.  One that gives up below is
-      // seen at the next check.
+      const double pq = total(s_pq);
       ok = s_fail == 0;
-      if (!ok) return;
-      // The team's z is there or about to be (each block stored it before its
-      // slot): read only now, so that early polls do not crowd the stores.
-      for (uint32_t e0 = 2u * tid; e0 < L; e0 += 2u * kInFlight * kTeamThreads) {
-        unsigned long long v[kInFlight][2];
-        const unsigned long long* w[kInFlight];
-#pragma unroll
-        for (int i = 0; i < kInFlight; ++i) {
-          const uint32_t e = min(e0 + i * 2u * kTeamThreads, L - 2u);
-          w[i] = zw + z_at[e / 2u];
-          get_words(w[i], v[i][0], v[i][1]);
-        }
-        Deadline dl;
-#pragma unroll
-        for (int i = 0; i < kInFlight; ++i) {
-          while (!fresh(v[i][0], epoch) || !fresh(v[i][1], epoch)) {
-            if (!dl.wait()) {
-              s_fail = 1;
-              break;
-            }
-            get_words(w[i], v[i][0], v[i][1]);
-          }
-          const uint32_t e = e0 + i * 2u * kTeamThreads;
-          if (e < L)
-            *reinterpret_cast<float2*>(z_in + e) =
-                make_float2(__uint_as_float((uint32_t)v[i][0]), __uint_as_float((uint32_t)v[i][1]));
-        }
+      if (!ok) break;
+      if (!(pq > 0.0) || !isfinite(pq)) {
+        status = 2;  // non-positive curvature: x unchanged
+        break;
       }
-      // Each thread updates the entries of p that it read: the next barrier
-      // is the one before the product.
-    };
-
-    exchange_z();
-    double rz = total(s_rz), rr = total(s_rr);
-    const LmParams& lp = d.params[P];
-    const double bnorm = sqrt(rr), stop = lp.pcg_relative_tolerance * bnorm;
-    // |r| <= stop without the root: on squares; a negative tolerance is never met.
-    const double stop2 = stop >= 0.0 ? stop * stop : -1.0;
-    const uint32_t cap = lp.max_pcg_iterations;
-    uint32_t iters = 0, status = 0;
-    // pcg_init (ba.wgsl:420-439): done when |b| = 0 or r.z <= 0.
-    if (ok && rr > 0.0 && rz > 0.0 && cap != 0u) {
-      float beta = 0.0f;
-      for (;;) {
-        const double inv_rz = inverse64(rz);
-        for (uint32_t e = 2u * tid; e < L; e += 2u * kTeamThreads) {
-          const float2 zv = *reinterpret_cast<const float2*>(z_in + e);
-          float2 pv = *reinterpret_cast<const float2*>(p + e);
-          pv.x = __fmaf_rn(beta, pv.x, zv.x);
-          pv.y = __fmaf_rn(beta, pv.y, zv.y);
-          *reinterpret_cast<float2*>(p + e) = pv;
-        }
-        po = __fmaf_rn(beta, po, z);
-        __syncthreads();
-        // Row sums of a part: the lanes' products by a reduce-scatter over
-        // bits 4 and 3, then a butterfly.
-        auto reduce = [&](const float (&acc)[6], uint32_t node, uint32_t seg, bool store) {
-          const bool b4 = (lane >> 4) & 1u, b3 = (lane >> 3) & 1u;
-          float h[3];
-#pragma unroll
-          for (int q = 0; q < 3; ++q) {
-            const float keep = b4 ? acc[q + 3] : acc[q], send = b4 ? acc[q] : acc[q + 3];
-            h[q] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-          }
-          const float g0 = __shfl_xor_sync(0xffffffffu, b3 ? h[0] : h[2], 8);
-          const float g1 = __shfl_xor_sync(0xffffffffu, h[1], 8);
-          float u = b3 ? h[2] + g0 : h[0] + g0, v = h[1] + g1;
-#pragma unroll
-          for (int off = 4; off > 0; off >>= 1) {
-            u += __shfl_xor_sync(0xffffffffu, u, off);
-            v += __shfl_xor_sync(0xffffffffu, v, off);
-          }
-          float* out = part + (size_t)seg * 6 * nn + 6 * node + (b4 ? 3 : 0);
-          if (store && (lane & 7u) == 0) out[b3 ? 2 : 0] = u;
-          if (store && (lane & 15u) == 1) out[1] = v;
-        };
-        auto madd = [](float4 s, float4 v, float& acc) {
-          acc = __fmaf_rn(s.x, v.x, acc);
-          acc = __fmaf_rn(s.y, v.y, acc);
-          acc = __fmaf_rn(s.z, v.z, acc);
-          acc = __fmaf_rn(s.w, v.w, acc);
-        };
-        const float4* p4 = reinterpret_cast<const float4*>(p);
-        // The held parts' products, then their reductions side by side (a
-        // part past the last holds zeros and stores nothing).
-        float held[kHeld][6];
-#pragma unroll
-        for (int u = 0; u < kHeld; ++u) {
-#pragma unroll
-          for (int q = 0; q < 6; ++q) held[u][q] = 0.0f;
-#pragma unroll
-          for (int j = 0; j < kSegVec; ++j) {
-            const float4 pv = p4[seg_held[u] * (kSegment / 4) + lane + 32 * j];
-#pragma unroll
-            for (int q = 0; q < 6; ++q) madd(Sr[u][q][j], pv, held[u][q]);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kHeld; ++u)
-          reduce(held[u], node_held[u], seg_held[u], warp + u * kTeamWarps < parts);
-        for (uint32_t it = kRegParts + warp; it < parts; it += kTeamWarps) {
-          const uint32_t node = it % nn, seg = it / nn;
-          const float4* s4 = reinterpret_cast<const float4*>(S + (size_t)(it - kRegParts) * kPartFloats);
-          float acc[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 1
-          for (int j = 0; j < kSegVec; ++j) {
-            const float4 pv = p4[seg * (kSegment / 4) + lane + 32 * j];
-#pragma unroll
-            for (int q = 0; q < 6; ++q) madd(s4[q * (kSegment / 4) + lane + 32 * j], pv, acc[q]);
-          }
-          reduce(acc, node, seg, true);
-        }
-        __syncthreads();
-        float qa = 0.0f;
-        if (own)
-          for (uint32_t s = 0; s < nseg; ++s) qa += part[(size_t)s * 6 * nn + 6 * gi + a];
-        ++epoch;
-        double pq_own = 0.0;
-        if (warp < nwarp) {
-          pq_own = warp_sum_t((double)po * (double)qa);
-          if (lane == 0) s_a[warp] = pq_own;
-        }
-        if (nwarp > 1) __syncthreads();
-        if (warp == 0) {
-          for (uint32_t w = 1; w < nwarp; ++w) pq_own += s_a[w];
-          if (lane < 2u)
-            put_word(pq_slots + kLineWords * T.rank + lane,
-                     (uint32_t)(lane ? __double2hiint(pq_own) : __double2loint(pq_own)), epoch);
-        }
-        if (32u * warp < T.size) {
-          double sum[1];
-          const bool got = gather_slots<1>(pq_slots, T.size, epoch, sum);
-          if (lane == 0) {
-            s_pq[warp] = sum[0];
-            if (!got) s_fail = 1;
-          }
-        }
-        __syncthreads();
-        const double pq = total(s_pq);
-        ok = s_fail == 0;
-        if (!ok) break;
-        if (!(pq > 0.0) || !isfinite(pq)) {
-          status = 2;  // non-positive curvature: x unchanged
-          break;
-        }
-        const float alpha = (float)(rz * inverse64(pq));
-        x = x + alpha * po;
-        r = r - alpha * qa;
-        exchange_z();
-        if (!ok) break;
-        const double rz_new = total(s_rz);
-        rr = total(s_rr);
-        ++iters;
-        rz = rz_new;
-        if (rr <= stop2 || !(rz_new > 0.0)) break;
-        if (iters >= cap) {
-          status = 1;
-          break;
-        }
-        beta = (float)(rz_new * inv_rz);
+      const float alpha = (float)(rz * inverse64(pq));
+      x = x + alpha * po;
+      r = r - alpha * qa;
+      exchange_z();
+      if (!ok) break;
+      const double rz_new = total(s_rz);
+      rr = total(s_rr);
+      ++iters;
+      rz = rz_new;
+      if (rr <= stop2 || !(rz_new > 0.0)) break;
+      if (iters >= cap) {
+        status = 1;
+        break;
       }
-    }
-    if (own) d.x[at] = x;
-    if (T.rank == 0 && tid == 0) {
-      PcgState& st = d.pcg[P];
-      st.iters = iters;
-      st.status = status;
-      st.bnorm = bnorm;
-      st.rnorm = sqrt(rr);
-      st.rz = rz;
-      st.active = 0u;
-      // Every block has read epoch0: this one has seen all their slots.  (A
-      // block that gave up is at most one exchange ahead of another.)
-      d.team_epoch[P] = epoch + 2u;
-    }
-    __syncthreads();
-    if (s_fail) {
-      if (tid == 0) atomicOr(d.error, (unsigned int)kErrBarrierTimeout);
-      return;
+      beta = (float)(rz_new * inv_rz);
     }
   }
+  if (own) d.x[at] = x;
+  if (T.rank == 0 && tid == 0) {
+    PcgState& st = d.pcg[P];
+    st.iters = iters;
+    st.status = status;
+    st.bnorm = bnorm;
+    st.rnorm = sqrt(rr);
+    st.rz = rz;
+    st.active = 0u;
+    // Every block has read epoch0: this one has seen all their slots.  (A
+    // block that gave up is at most one exchange ahead of another.)
+    d.team_epoch[P] = epoch + 2u;
+  }
+  __syncthreads();
+  if (s_fail && tid == 0) atomicOr(d.error, (unsigned int)kErrBarrierTimeout);
 }
 
 uint32_t team_parts(uint32_t nodes, uint32_t ncols) {
@@ -570,21 +562,15 @@ TeamPlan build_team_plan(const uint32_t* prob_tr_begin, uint32_t num_problems,
     teams.push_back(Team{first, size});
   }
   // Rounds of teams that fit the device together, in problem order.
-  std::vector<std::vector<uint32_t>> rounds;
   uint32_t used = 0;
   for (const Team& t : teams) {
-    if (rounds.empty() || used + t.size > max_blocks) {
-      rounds.emplace_back();
+    if (tp.round_begin.empty() || used + t.size > max_blocks) {
+      tp.round_begin.push_back(t.first);
       used = 0;
     }
-    for (uint32_t g = 0; g < t.size; ++g) rounds.back().push_back(t.first + g);
     used += t.size;
-    tp.grid = std::max(tp.grid, used);
   }
-  tp.rounds = (uint32_t)rounds.size();
-  tp.sched.assign((size_t)tp.rounds * tp.grid, kNone);
-  for (size_t r = 0; r < rounds.size(); ++r)
-    std::copy(rounds[r].begin(), rounds[r].end(), tp.sched.begin() + (long)(r * tp.grid));
+  if (!teams.empty()) tp.round_begin.push_back((uint32_t)tp.cta.size());
   return tp;
 }
 
@@ -593,9 +579,17 @@ cudaError_t launch_pcg_team(const Dev& d, cudaStream_t s) {
   const cudaError_t e = cudaFuncSetAttribute(
       k_pcg_team, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d.team_smem);
   if (e != cudaSuccess) return e;
-  void* args[] = {const_cast<Dev*>(&d)};
-  return cudaLaunchCooperativeKernel((const void*)k_pcg_team, d.team_grid, kTeamThreads, args,
-                                     d.team_smem, s);
+  // A launch a round: in one launch over all of them a block waited for the
+  // teammates of its next round while they still solved the last one, as long
+  // as that solve took, under the limit of a wait.
+  for (uint32_t r = 0; r < d.team_rounds; ++r) {
+    uint32_t first = d.team_round_begin[r];
+    void* args[] = {const_cast<Dev*>(&d), &first};
+    const cudaError_t l = cudaLaunchCooperativeKernel(
+        (const void*)k_pcg_team, d.team_round_begin[r + 1] - first, kTeamThreads, args, d.team_smem, s);
+    if (l != cudaSuccess) return l;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace vlba

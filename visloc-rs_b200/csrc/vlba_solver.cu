@@ -211,6 +211,7 @@ struct Context {
   uint32_t flags = 0;  // flags of the uploaded config
   size_t l2_bytes = 0;
   double l2_fraction = 0.5;  // share of the L2 that keeps S resident in PCG
+  std::vector<uint32_t> team_round_begin;  // Dev::team_round_begin
   int pcg_grid_hint = 0;     // blocks of the PCG launch (trace sizing)
   // the uploaded problems' sizes (for download)
   std::vector<uint64_t> num_poses, num_points;
@@ -507,7 +508,7 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
   d.small_list = st.up(A, small);
   // Then the problems that fit a team of blocks; the persistent kernel has
   // the rest.
-  const TeamPlan team = build_team_plan(P.prob_tr_begin.data(), P.num_problems, P.tile_ij, tile_begin,
+  TeamPlan team = build_team_plan(P.prob_tr_begin.data(), P.num_problems, P.tile_ij, tile_begin,
                                         (uint32_t)c->sm_count);
   std::vector<uint8_t> big(P.num_problems, 0);
   for (uint32_t p = 0; p < P.num_problems; ++p) {
@@ -525,15 +526,15 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
   }
   for (uint32_t& n : long_terms) n = long_block_terms(n);
   d.prob_long_terms = st.up(A, long_terms);
-  d.team_rounds = team.rounds;
-  d.team_grid = team.grid;
+  c->team_round_begin = std::move(team.round_begin);
+  d.team_rounds = c->team_round_begin.empty() ? 0u : (uint32_t)c->team_round_begin.size() - 1;
+  d.team_round_begin = c->team_round_begin.data();
   d.team_smem = (uint32_t)team.smem;
   d.team_slots_total = (uint32_t)team.cta.size();
   d.team_cta = st.up(A, team.cta);
-  d.team_sched = st.up(A, team.sched);
   d.team_cols = st.up(A, team.cols);
   d.team_ents = st.up(A, team.ents);
-  if (team.rounds) {
+  if (d.team_rounds) {
     // Number 0 is no exchange's.
     const size_t words = team.z_words + 2 * kLineWords * team.cta.size();
     d.team_z = A.alloc<unsigned long long>(words);
@@ -818,7 +819,7 @@ void dump_trace(Context* c) {
 // the PCG kernels when the system has them.
 uint64_t iteration_launches(const Dev& d) {
   uint64_t n = 5 + (d.num_offdiag_blocks > d.num_long_blocks ? 1 : 0) + (d.num_long_blocks ? 1 : 0) +
-               (d.num_var_cams ? 1 : 0) + (d.team_rounds ? 1 : 0) + (d.num_big ? 2 : 0);
+               (d.num_var_cams ? 1 : 0) + d.team_rounds + (d.num_big ? 2 : 0);
   for (int k = 0; k < kSmallPcgClasses; ++k) n += d.small_off[k + 1] > d.small_off[k] ? 1 : 0;
   return n;
 }
