@@ -567,8 +567,10 @@ const char* visloc_ba_cuda_server_last_error(void* server);
  * row counters, the grid barrier give up after 2 s, set an error bit and let
  * the kernel return, so a lost arrival becomes VLBA_ERR_TIMEOUT instead of a
  * hung GPU): waits on a device flag that nothing sets for limit_ms and
- * returns VLBA_ERR_TIMEOUT with the time it waited.  The context stays usable
- * afterwards.  No reference counterpart. */
+ * returns VLBA_ERR_TIMEOUT with the time it waited.  With an upload whose
+ * systems are solved by teams of blocks, also runs the first teams without
+ * one of their blocks, under the same limit.  The context and its upload stay
+ * usable afterwards, and the state of the last solve stays as it is.  No reference counterpart. */
 int visloc_ba_cuda_wait_probe(void* ctx, double limit_ms, double* waited_ms);
 
 /* One damped linear step at the given state, without updating it: the step

@@ -47,6 +47,11 @@ TeamPlan build_team_plan(const uint32_t* prob_tr_begin, uint32_t num_problems,
                          const std::vector<uint32_t>& tile_ij,
                          const std::vector<uint32_t>& tile_begin, uint32_t max_blocks);
 cudaError_t launch_pcg_team(const Dev& d, cudaStream_t s);
+// Self-test of the teams' waits: the first round without its first block, whose
+// teammates give up after limit_ns (kErrBarrierTimeout in d.error).
+cudaError_t launch_team_probe(const Dev& d, unsigned long long limit_ns, cudaStream_t s);
+// The exchange words and numbers as after an upload.
+cudaError_t clear_team_words(const Dev& d, cudaStream_t s);
 cudaError_t launch_pose_update(const Dev& d, cudaStream_t s);
 // Fill the tiles, preconditioner and rhs of a reduced system given directly
 // (device arrays in the reference's layout; the off-diagonal blocks f32, or

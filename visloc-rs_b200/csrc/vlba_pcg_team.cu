@@ -22,7 +22,8 @@
 // written again only after its writer has seen every block's slot of the
 // exchange in between, which each block publishes after its own reads.  The
 // numbers go on from one solve to the next (team_epoch), so what an earlier
-// solve left is never taken for news.  A slot, and a block's z, has its 128-byte
+// solve left is never taken for news (after a wait that gave up, whose blocks
+// may have stopped at different numbers, the host clears words and numbers).  A slot, and a block's z, has its 128-byte
 // lines to itself: with eight slots a line, polled by a hundred blocks while
 // eight write, an exchange took 3,800 cycles of 148 blocks, alone in a line
 // 1,800 (a counter barrier with loads behind it: 3,000).
@@ -85,12 +86,13 @@ __device__ __forceinline__ double join(unsigned long long lo, unsigned long long
 // Bounded polling: true while the deadline is ahead (the timer, slow to read,
 // only every 256 misses).
 struct Deadline {
+  unsigned long long limit_ns;
   unsigned long long t_end = 0;
   uint32_t misses = 0;
   __device__ __forceinline__ bool wait() {
     if ((++misses & 255u) != 0u) return true;
     const unsigned long long t = now_ns();
-    if (t_end == 0) t_end = t + kWaitLimitNs;
+    if (t_end == 0) t_end = t + limit_ns;
     return t <= t_end;
   }
 };
@@ -99,14 +101,15 @@ struct Deadline {
 // fixed order; false when a slot never came.
 template <int V>
 __device__ __forceinline__ bool gather_slots(const unsigned long long* slots, uint32_t size,
-                                             uint32_t epoch, double (&sum)[V]) {
+                                             uint32_t epoch, unsigned long long limit_ns,
+                                             double (&sum)[V]) {
   const uint32_t g = threadIdx.x;  // warp w has slots 32 w to 32 w + 31
   unsigned long long w[2 * V];
   bool ok = true;
 #pragma unroll
   for (int v = 0; v < 2 * V; ++v) w[v] = (unsigned long long)epoch << 32;
   if (g < size) {
-    Deadline dl;
+    Deadline dl{limit_ns};
     for (;;) {
       bool miss = false;
 #pragma unroll
@@ -126,7 +129,9 @@ __device__ __forceinline__ bool gather_slots(const unsigned long long* slots, ui
   return ok;
 }
 
-__global__ void __launch_bounds__(kTeamThreads, 1) k_pcg_team(Dev d, uint32_t first) {
+// Block `absent` (kNone: none) stays out, for the test of the waits.
+__global__ void __launch_bounds__(kTeamThreads, 1) k_pcg_team(Dev d, uint32_t first, uint32_t absent,
+                                                              unsigned long long limit_ns) {
   extern __shared__ __align__(16) float smem[];
   __shared__ double s_a[kTeamWarps], s_b[kTeamWarps], s_rz[kTeamPolls], s_rr[kTeamPolls],
       s_pq[kTeamPolls];
@@ -136,6 +141,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pcg_team(Dev d, uint32_t fi
   const TeamCta T = d.team_cta[first + blockIdx.x];
   const uint32_t P = T.prob;
   if (d.ctrl[P].done) return;  // the same for the whole team
+  if (blockIdx.x == absent) return;
   const uint32_t nn = T.node1 - T.node0, L = 48u * T.ncols, nseg = (T.ncols + kSegTiles - 1) / kSegTiles;
   const uint32_t parts = nn * nseg, Lp = nseg * kSegment;
   const uint32_t tr0 = d.prob_tr_begin[P], slot0 = 8u * tr0;
@@ -262,7 +268,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pcg_team(Dev d, uint32_t fi
     }
     if (32u * warp < T.size) {
       double sum[2];
-      const bool got = gather_slots<2>(rz_slots, T.size, epoch, sum);
+      const bool got = gather_slots<2>(rz_slots, T.size, epoch, limit_ns, sum);
       if (lane == 0) {
         s_rz[warp] = sum[0];
         s_rr[warp] = sum[1];
@@ -270,7 +276,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pcg_team(Dev d, uint32_t fi
       }
     }
     __syncthreads();
-    // A wait that gives up has lasted kWaitLimitNs: no thread sets s_fail
+    // A wait that gives up has lasted limit_ns: no thread sets s_fail
     // while another is still on its way here.  One that gives up below is
     // seen at the next check.
     ok = s_fail == 0;
@@ -286,7 +292,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pcg_team(Dev d, uint32_t fi
         w[i] = zw + z_at[e / 2u];
         get_words(w[i], v[i][0], v[i][1]);
       }
-      Deadline dl;
+      Deadline dl{limit_ns};
 #pragma unroll
       for (int i = 0; i < kInFlight; ++i) {
         while (!fresh(v[i][0], epoch) || !fresh(v[i][1], epoch)) {
@@ -405,7 +411,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pcg_team(Dev d, uint32_t fi
       }
       if (32u * warp < T.size) {
         double sum[1];
-        const bool got = gather_slots<1>(pq_slots, T.size, epoch, sum);
+        const bool got = gather_slots<1>(pq_slots, T.size, epoch, limit_ns, sum);
         if (lane == 0) {
           s_pq[warp] = sum[0];
           if (!got) s_fail = 1;
@@ -574,22 +580,37 @@ TeamPlan build_team_plan(const uint32_t* prob_tr_begin, uint32_t num_problems,
   return tp;
 }
 
-cudaError_t launch_pcg_team(const Dev& d, cudaStream_t s) {
-  if (d.team_rounds == 0) return cudaSuccess;
+static cudaError_t launch_round(const Dev& d, uint32_t round, uint32_t absent,
+                                unsigned long long limit_ns, cudaStream_t s) {
   const cudaError_t e = cudaFuncSetAttribute(
       k_pcg_team, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d.team_smem);
   if (e != cudaSuccess) return e;
+  uint32_t first = d.team_round_begin[round];
+  void* args[] = {const_cast<Dev*>(&d), &first, &absent, &limit_ns};
+  return cudaLaunchCooperativeKernel((const void*)k_pcg_team, d.team_round_begin[round + 1] - first,
+                                     kTeamThreads, args, d.team_smem, s);
+}
+
+cudaError_t launch_pcg_team(const Dev& d, cudaStream_t s) {
   // A launch a round: in one launch over all of them a block waited for the
   // teammates of its next round while they still solved the last one, as long
   // as that solve took, under the limit of a wait.
-  for (uint32_t r = 0; r < d.team_rounds; ++r) {
-    uint32_t first = d.team_round_begin[r];
-    void* args[] = {const_cast<Dev*>(&d), &first};
-    const cudaError_t l = cudaLaunchCooperativeKernel(
-        (const void*)k_pcg_team, d.team_round_begin[r + 1] - first, kTeamThreads, args, d.team_smem, s);
-    if (l != cudaSuccess) return l;
-  }
-  return cudaSuccess;
+  cudaError_t e = cudaSuccess;
+  for (uint32_t r = 0; r < d.team_rounds && e == cudaSuccess; ++r)
+    e = launch_round(d, r, kNone, kWaitLimitNs, s);
+  return e;
+}
+
+cudaError_t launch_team_probe(const Dev& d, unsigned long long limit_ns, cudaStream_t s) {
+  return launch_round(d, 0, 0u, limit_ns, s);
+}
+
+cudaError_t clear_team_words(const Dev& d, cudaStream_t s) {
+  if (d.team_rounds == 0) return cudaSuccess;
+  // The slots follow the z words.
+  const size_t words = (size_t)(d.team_slots - d.team_z) + 2 * kLineWords * (size_t)d.team_slots_total;
+  const cudaError_t e = cudaMemsetAsync(d.team_z, 0, 8 * words, s);
+  return e != cudaSuccess ? e : cudaMemsetAsync(d.team_epoch, 0, 4 * (size_t)d.num_problems, s);
 }
 
 }  // namespace vlba

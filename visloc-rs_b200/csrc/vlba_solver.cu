@@ -536,12 +536,10 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
   d.team_ents = st.up(A, team.ents);
   if (d.team_rounds) {
     // Number 0 is no exchange's.
-    const size_t words = team.z_words + 2 * kLineWords * team.cta.size();
-    d.team_z = A.alloc<unsigned long long>(words);
+    d.team_z = A.alloc<unsigned long long>(team.z_words + 2 * kLineWords * team.cta.size());
     d.team_slots = d.team_z + team.z_words;
     d.team_epoch = A.alloc<uint32_t>(P.num_problems);
-    VLBA_CUDA(cudaMemsetAsync(d.team_z, 0, 8 * words, s));
-    VLBA_CUDA(cudaMemsetAsync(d.team_epoch, 0, 4 * (size_t)P.num_problems, s));
+    check_launch(clear_team_words(d, s), "team words");
   }
   d.pose_prob = st.up(A, P.pose_prob);
   d.point_prob = st.up(A, P.point_prob);
@@ -868,13 +866,21 @@ uint64_t enqueue_initial(Context* c) {
   return 3;
 }
 
+// A device wait gave up (its error bits): waits for what is still in flight and
+// clears the teams' words, some of which may carry numbers that the next solve
+// would take for its own.
+[[noreturn]] void wait_gave_up(Context* c, unsigned int err) {
+  check_launch(clear_team_words(c->dev, c->stream), "team words");
+  VLBA_CUDA(cudaStreamSynchronize(c->stream));
+  throw Status(VLBA_ERR_TIMEOUT,
+               "a bounded device wait gave up (error bits " + std::to_string(err) + ")");
+}
+
 void check_device_error(Context* c) {
   unsigned int err = 0;
   VLBA_CUDA(cudaMemcpyAsync(&err, c->dev.error, 4, cudaMemcpyDeviceToHost, c->stream));
   VLBA_CUDA(cudaStreamSynchronize(c->stream));
-  if (err)
-    throw Status(VLBA_ERR_TIMEOUT,
-                 "a bounded device wait gave up (error bits " + std::to_string(err) + ")");
+  if (err) wait_gave_up(c, err);
 }
 
 // The LM loop with VLBA_FLAG_GRAPH: the initial cost and max_iters
@@ -939,11 +945,7 @@ RunStats run_lm(Context* c, bool profile, PhaseTimes* pt) {
   volatile unsigned int* const state = c->host_state;  // written by k_decide
   state[0] = state[1] = 0u;
   auto check_error = [&] {
-    if (const unsigned int err = state[1]) {
-      VLBA_CUDA(cudaStreamSynchronize(s));
-      throw Status(VLBA_ERR_TIMEOUT,
-                   "a bounded device wait gave up (error bits " + std::to_string(err) + ")");
-    }
+    if (const unsigned int err = state[1]) wait_gave_up(c, err);
   };
   VLBA_CUDA(cudaEventRecord(c->ev[0], s));
   st.launches += enqueue_initial(c);
@@ -1892,7 +1894,7 @@ int visloc_ba_cuda_linear_step(void* ctx, const vlba_problem* problem, const vlb
     unsigned int err = 0;
     VLBA_CUDA(cudaMemcpyAsync(&err, d.error, 4, cudaMemcpyDeviceToHost, s));
     VLBA_CUDA(cudaStreamSynchronize(s));
-    if (err) throw vlba::Status(VLBA_ERR_TIMEOUT, "a bounded device wait gave up");
+    if (err) vlba::wait_gave_up(c, err);
     if (dp) {
       size_t n = 0;
       for (size_t i = 0; i < P.pose_slot.size(); ++i)
@@ -2779,7 +2781,7 @@ int visloc_ba_cuda_reduced_solve(void* ctx, const vlba_reduced_system* sys, doub
     unsigned int err = 0;
     VLBA_CUDA(cudaMemcpyAsync(&err, d.error, 4, cudaMemcpyDeviceToHost, s));
     VLBA_CUDA(cudaStreamSynchronize(s));
-    if (err) throw vlba::Status(VLBA_ERR_TIMEOUT, "a bounded device wait gave up");
+    if (err) vlba::wait_gave_up(c, err);
     vlba::download_step(c, sys->num_nodes, x);
     if (iterations) *iterations = pg.iters;
     if (relative_residual) *relative_residual = pg.bnorm > 0 ? pg.rnorm / pg.bnorm : 0.0;
@@ -2864,6 +2866,23 @@ int visloc_ba_cuda_wait_probe(void* ctx, double limit_ms, double* waited_ms) {
     VLBA_CUDA(cudaMemcpyAsync(&ns, waited, 8, cudaMemcpyDeviceToHost, c->stream));
     VLBA_CUDA(cudaStreamSynchronize(c->stream));
     if (waited_ms) *waited_ms = ns / 1e6;
+    // The teams' waits, where the upload has teams, on the system as it is
+    // there; the control words (a finished problem's blocks return at once)
+    // are put back.
+    if (!err || !c->uploaded || c->dev.team_rounds == 0) return;
+    const vlba::Dev& d = c->dev;
+    const size_t bytes = sizeof(vlba::Ctrl) * d.num_problems;
+    std::vector<vlba::Ctrl> ctrl(d.num_problems);
+    VLBA_CUDA(cudaMemcpyAsync(ctrl.data(), d.ctrl, bytes, cudaMemcpyDeviceToHost, c->stream));
+    VLBA_CUDA(cudaMemsetAsync(d.ctrl, 0, bytes, c->stream));
+    VLBA_CUDA(cudaMemsetAsync(d.error, 0, 8, c->stream));
+    vlba::check_launch(vlba::launch_team_probe(d, (unsigned long long)(limit_ms * 1e6), c->stream),
+                       "team wait probe");
+    VLBA_CUDA(cudaMemcpyAsync(&err, d.error, 4, cudaMemcpyDeviceToHost, c->stream));
+    VLBA_CUDA(cudaMemsetAsync(d.error, 0, 8, c->stream));
+    VLBA_CUDA(cudaMemcpyAsync(d.ctrl, ctrl.data(), bytes, cudaMemcpyHostToDevice, c->stream));
+    VLBA_CUDA(cudaStreamSynchronize(c->stream));
+    if (err) vlba::wait_gave_up(c, err);
   });
   if (st != VLBA_OK) return st;
   if (err) {
