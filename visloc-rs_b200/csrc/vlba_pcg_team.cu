@@ -61,6 +61,11 @@ constexpr uint32_t kSegTiles = 8, kSegment = 48 * kSegTiles;  // columns of a pa
 constexpr int kSegVec = kSegment / 128;               // float4 per lane and row
 constexpr uint32_t kPartFloats = 6 * kSegment;
 constexpr uint32_t kExtra = 22;                       // parts kept in shared memory
+// Dynamic shared memory a block may take: sm_100's 227 KB less the static
+// arrays.  The launch attribute is always set to it, whatever a plan needs: it
+// belongs to the kernel, and another thread's smaller plan set it below what
+// this one was about to launch with.
+constexpr size_t kTeamMaxSmem = (227 - 1) * 1024;
 
 __device__ __forceinline__ double warp_sum_t(double v) {
 #pragma unroll
@@ -472,8 +477,9 @@ size_t team_smem(uint32_t nodes, uint32_t ncols) {
 }  // namespace
 
 // Blocks of one problem for a team of `size`; the most parts of a block (its
-// bytes in *smem), or 0 when a block would own or read too many cameras.  `near` lists each tile row's
-// columns (both triangles), ascending.
+// bytes in *smem), or 0 when a block would own or read too many cameras or not
+// fit its shared memory.  `near` lists each tile row's columns (both triangles),
+// ascending.
 static uint32_t split_team(const std::vector<std::vector<uint32_t>>& near, uint32_t size,
                            std::vector<TeamCta>* out, std::vector<uint32_t>* cols, size_t* smem) {
   const uint32_t R = (uint32_t)near.size(), nodes = 8 * R;
@@ -496,7 +502,9 @@ static uint32_t split_team(const std::vector<std::vector<uint32_t>>& near, uint3
     T.ncols = (uint32_t)u.size();
     if (T.ncols > kTeamMaxCols) return 0;
     worst = std::max(worst, team_parts(T.node1 - T.node0, T.ncols));
-    *smem = std::max(*smem, team_smem(T.node1 - T.node0, T.ncols));
+    const size_t bytes = team_smem(T.node1 - T.node0, T.ncols);
+    if (bytes > kTeamMaxSmem) return 0;
+    *smem = std::max(*smem, bytes);
     if (out) {
       T.col_begin = (uint32_t)cols->size();
       cols->insert(cols->end(), u.begin(), u.end());
@@ -583,7 +591,7 @@ TeamPlan build_team_plan(const uint32_t* prob_tr_begin, uint32_t num_problems,
 static cudaError_t launch_round(const Dev& d, uint32_t round, uint32_t absent,
                                 unsigned long long limit_ns, cudaStream_t s) {
   const cudaError_t e = cudaFuncSetAttribute(
-      k_pcg_team, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d.team_smem);
+      k_pcg_team, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTeamMaxSmem);
   if (e != cudaSuccess) return e;
   uint32_t first = d.team_round_begin[round];
   void* args[] = {const_cast<Dev*>(&d), &first, &absent, &limit_ns};
