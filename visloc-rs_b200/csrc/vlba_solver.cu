@@ -931,7 +931,23 @@ RunStats run_lm_graph(Context* c, uint32_t max_iters) {
 
 LaunchShape autotune(Context* c);
 
+// A solve that ends by an exception leaves nothing in flight: an iteration
+// issued ahead would set the done flag of the next solve (host_state) after
+// that solve has cleared it.  A timeout may then be unreported, so the teams'
+// words are cleared too.
+struct SettleOnThrow {
+  Context* c;
+  int exceptions = std::uncaught_exceptions();
+  ~SettleOnThrow() {
+    if (std::uncaught_exceptions() <= exceptions) return;
+    cudaStreamSynchronize(c->side);
+    clear_team_words(c->dev, c->stream);
+    cudaStreamSynchronize(c->stream);
+  }
+};
+
 RunStats run_lm(Context* c, bool profile, PhaseTimes* pt) {
+  const SettleOnThrow settle{c};
   if ((c->flags & VLBA_FLAG_AUTOTUNE) && !c->tuned) {
     autotune(c);
     reset_state(c);
