@@ -177,3 +177,18 @@ def test_each_round_of_teams_is_a_launch(solver):
     assert statuses == [0, 0]
     assert both[0].kernel_launches == alone.kernel_launches + 2
     assert both[0].final_cost == both[1].final_cost == alone.final_cost
+
+
+def test_the_phase_trace_covers_the_persistent_kernel_only(solver, monkeypatch, capfd):
+    """VLBA_TRACE_PCG prints what k_pcg measured, and nothing for systems that
+    it does not solve (their trace memory holds nothing)."""
+    monkeypatch.setenv("VLBA_TRACE_PCG", "1")
+    cfg = BaConfig(max_iterations=2, max_pcg_iterations=12)
+    small, big = synth.ring_problem(20, 800, seed=1), synth.ring_problem(620, 24800, seed=2)
+    statuses, _ = solver.batch_optimize([small.copy(), synth.ring_problem(140, 5600, seed=3)], cfg)
+    assert statuses == [0, 0] and capfd.readouterr().err == ""
+    statuses, results = solver.batch_optimize([small.copy(), big.copy()], cfg)
+    assert statuses == [0, 0]
+    lines = [s for s in capfd.readouterr().err.splitlines() if s.startswith("vlba pcg trace:")]
+    assert [int(s.split()[3]) for s in lines] == [i.pcg_iterations for i in results[1].iterations]
+    assert all(0.0 < float(s.split()[-1]) < 1e4 for s in lines)

@@ -761,17 +761,29 @@ struct PhaseTimes {
   std::vector<double> lin, assemble, pcg, update;
 };
 
-// VLBA_TRACE_PCG: per-phase device time of the PCG iterations (mean over
-// blocks of each phase's span, and the iteration's wall span), to stderr.
+// VLBA_TRACE_PCG: per-phase device time of the persistent kernel's iterations
+// (mean over blocks of each phase's span, and the iteration's wall span), to
+// stderr; nothing where that kernel solves no problem of the upload.
 void dump_trace(Context* c) {
   const Dev& d = c->dev;
+  if (d.num_big == 0) return;
   const int G = c->pcg_grid;
   std::vector<unsigned long long> t((size_t)kTraceIters * G * kTracePhases);
   VLBA_CUDA(cudaMemcpyAsync(t.data(), d.trace, t.size() * 8, cudaMemcpyDeviceToHost, c->stream));
-  PcgState pg;
-  VLBA_CUDA(cudaMemcpyAsync(&pg, d.pcg, sizeof pg, cudaMemcpyDeviceToHost, c->stream));
+  std::vector<PcgState> pg(d.num_problems);
+  std::vector<Ctrl> ctrl(d.num_problems);
+  std::vector<uint8_t> big(d.num_problems);
+  VLBA_CUDA(cudaMemcpyAsync(pg.data(), d.pcg, pg.size() * sizeof(PcgState), cudaMemcpyDeviceToHost,
+                            c->stream));
+  VLBA_CUDA(cudaMemcpyAsync(ctrl.data(), d.ctrl, ctrl.size() * sizeof(Ctrl), cudaMemcpyDeviceToHost,
+                            c->stream));
+  VLBA_CUDA(cudaMemcpyAsync(big.data(), d.prob_big, big.size(), cudaMemcpyDeviceToHost, c->stream));
   VLBA_CUDA(cudaStreamSynchronize(c->stream));
-  const int iters = std::min<int>((int)pg.iters, kTraceIters - 1);
+  // The launch ran as long as its slowest problem.
+  uint32_t most = 0;
+  for (size_t p = 0; p < pg.size(); ++p)
+    if (big[p] && !ctrl[p].done) most = std::max(most, pg[p].iters);
+  const int iters = std::min<int>((int)most, kTraceIters - 1);
   double acc[kTracePhases] = {0};
   double wall = 0.0;
   for (int k = 0; k < iters; ++k) {
@@ -808,7 +820,7 @@ void dump_trace(Context* c) {
     std::fprintf(stderr,
                  "vlba pcg trace: %u iterations, per iteration (us): status %.2f tiles %.2f "
                  "arrive+reduce %.2f barrier1 %.2f update %.2f barrier2 %.2f | span %.2f\n",
-                 pg.iters, acc[1] / iters / 1e3, acc[2] / iters / 1e3, 0.0, acc[3] / iters / 1e3,
+                 most, acc[1] / iters / 1e3, acc[2] / iters / 1e3, 0.0, acc[3] / iters / 1e3,
                  acc[4] / iters / 1e3, acc[5] / iters / 1e3, wall / iters / 1e3);
 }
 
