@@ -192,3 +192,19 @@ def test_the_phase_trace_covers_the_persistent_kernel_only(solver, monkeypatch, 
     lines = [s for s in capfd.readouterr().err.splitlines() if s.startswith("vlba pcg trace:")]
     assert [int(s.split()[3]) for s in lines] == [i.pcg_iterations for i in results[1].iterations]
     assert all(0.0 < float(s.split()[-1]) < 1e4 for s in lines)
+
+
+@pytest.mark.parametrize("cluster", [1, 8])
+def test_without_large_clusters_the_teams_take_over(cluster, monkeypatch):
+    """On a device that places no cluster of 16 (or 4) blocks, the systems
+    those solve go to a team of blocks."""
+    from visloc_ba.solver import CudaSolver
+
+    monkeypatch.setenv("VLBA_MAX_CLUSTER", str(cluster))
+    with CudaSolver(0) as s:
+        for n in (17, 33, 40, 64, 65, 100, 128):
+            diag, edges, off, rhs = system(n, 0.6, n)
+            x, it, _ = s.reduced_solve(diag, edges, off, rhs, 0.0, 3)
+            ref, _ = pcg64(dense(diag, edges, off), diag, rhs, -1.0, 3)
+            assert it == 3
+            assert np.linalg.norm(x.reshape(-1) - ref) <= 1e-5 * np.linalg.norm(ref)

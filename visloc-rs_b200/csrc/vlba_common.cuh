@@ -121,9 +121,11 @@ inline __host__ __device__ uint32_t long_block_terms(uint32_t problem_blocks) {
 }
 constexpr int kLongLanes = 32;
 
-// Problems of at most this many tile rows (128 cameras) are solved by the
-// cluster kernels of vlba_pcg_small.cu, the others by the persistent k_pcg; a
-// problem's kernel follows from its own size, the same alone and in any batch.
+// Problems of at most this many tile rows (128 cameras; 64 where the device
+// places no cluster of 16 blocks, see small_pcg_rows) are solved by the cluster
+// kernels of vlba_pcg_small.cu, the others by a team of blocks
+// (vlba_pcg_team.cu) or the persistent k_pcg; a problem's kernel follows from
+// its own size, the same alone and in any batch.
 constexpr uint32_t kSmallPcgRows = 16;
 constexpr int kSmallPcgClasses = 4;
 

@@ -32,8 +32,11 @@ cudaError_t launch_pcg(const Dev& d, int grid, cudaStream_t s);
 cudaError_t launch_pcg_small(const Dev& d, cudaStream_t s);
 // Class of a problem of `rows` tile rows, or -1 for a larger one.
 int small_pcg_class(uint32_t rows);
+// The most tile rows whose class the current device can place with clusters of
+// at most max_cluster blocks.
+uint32_t small_pcg_rows(uint32_t max_cluster);
 
-// The problems past the small classes whose S fits the shared memory of a team
+// The problems of more than small_rows tile rows whose S fits the shared memory of a team
 // of blocks (vlba_pcg_team.cu): the teams' blocks, and the rounds of teams that
 // fit the device together (round r: blocks round_begin[r] to round_begin[r + 1]).
 struct TeamPlan {
@@ -45,7 +48,8 @@ struct TeamPlan {
 };
 TeamPlan build_team_plan(const uint32_t* prob_tr_begin, uint32_t num_problems,
                          const std::vector<uint32_t>& tile_ij,
-                         const std::vector<uint32_t>& tile_begin, uint32_t max_blocks);
+                         const std::vector<uint32_t>& tile_begin, uint32_t small_rows,
+                         uint32_t max_blocks);
 cudaError_t launch_pcg_team(const Dev& d, cudaStream_t s);
 // Self-test of the teams' waits: the first round without its first block, whose
 // teammates give up after limit_ns (kErrBarrierTimeout in d.error).

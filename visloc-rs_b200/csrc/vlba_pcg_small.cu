@@ -313,27 +313,47 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
   }
 }
 
+// The launch of a class's kernel on `problems` clusters of C blocks.
+template <int C, int W, int CPL, int N>
+struct ClassLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cudaError_t error = cudaSuccess;
+  ClassLaunch(uint32_t problems, cudaStream_t s) {
+    if (C > 8)  // beyond the portable cluster size
+      error = cudaFuncSetAttribute(k_pcg_small<C, W, CPL, N>,
+                                   cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cfg.gridDim = dim3(C * problems);
+    cfg.blockDim = dim3(32 * W);
+    cfg.stream = s;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = C > 1 ? 1 : 0;
+  }
+};
+
 template <int C, int W, int CPL, int N>
 cudaError_t launch_class(const Dev& d, uint32_t begin, uint32_t end, cudaStream_t s) {
   if (begin == end) return cudaSuccess;
-  auto kernel = k_pcg_small<C, W, CPL, N>;
-  if (C > 8) {  // beyond the portable cluster size
-    const cudaError_t e =
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(C * (end - begin));
-  cfg.blockDim = dim3(32 * W);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = C;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = C > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, d, d.small_list + begin);
+  const ClassLaunch<C, W, CPL, N> l(end - begin, s);
+  if (l.error != cudaSuccess) return l.error;
+  return cudaLaunchKernelEx(&l.cfg, k_pcg_small<C, W, CPL, N>, d, d.small_list + begin);
+}
+
+// Whether the device can place one of the class's clusters (a partition of it
+// may have no 16 SMs in one GPC).
+template <int C, int W, int CPL, int N>
+bool class_fits() {
+  const ClassLaunch<C, W, CPL, N> l(1, nullptr);
+  int clusters = 0;
+  const bool ok = l.error == cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&clusters, k_pcg_small<C, W, CPL, N>, &l.cfg) ==
+                      cudaSuccess;
+  cudaGetLastError();
+  return ok && clusters > 0;
 }
 
 }  // namespace
@@ -344,6 +364,11 @@ int small_pcg_class(uint32_t rows) {
   if (rows <= 8) return 2;
   if (rows <= kSmallPcgRows) return 3;
   return -1;
+}
+
+uint32_t small_pcg_rows(uint32_t max_cluster) {
+  if (max_cluster < 4 || !class_fits<4, 16, 12, 1>()) return 4;
+  return max_cluster < 16 || !class_fits<16, 8, 24, 1>() ? 8 : kSmallPcgRows;
 }
 
 cudaError_t launch_pcg_small(const Dev& d, cudaStream_t s) {

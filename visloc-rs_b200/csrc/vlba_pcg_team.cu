@@ -516,7 +516,8 @@ static uint32_t split_team(const std::vector<std::vector<uint32_t>>& near, uint3
 
 TeamPlan build_team_plan(const uint32_t* prob_tr_begin, uint32_t num_problems,
                          const std::vector<uint32_t>& tile_ij,
-                         const std::vector<uint32_t>& tile_begin, uint32_t max_blocks) {
+                         const std::vector<uint32_t>& tile_begin, uint32_t small_rows,
+                         uint32_t max_blocks) {
   TeamPlan tp;
   tp.in_team.assign(num_problems, 0);
   max_blocks = std::min(max_blocks, kTeamBlocks);
@@ -526,7 +527,7 @@ TeamPlan build_team_plan(const uint32_t* prob_tr_begin, uint32_t num_problems,
   std::vector<Team> teams;
   for (uint32_t p = 0; p < num_problems; ++p) {
     const uint32_t tr0 = prob_tr_begin[p], R = prob_tr_begin[p + 1] - tr0;
-    if (R <= kSmallPcgRows) continue;
+    if (R <= small_rows) continue;
     const uint32_t most = kRegParts + kExtra;
     const uint64_t tiles = tile_begin[p + 1] - tile_begin[p];
     if ((2 * tiles - R) * 8 / kSegTiles > (uint64_t)max_blocks * most) continue;  // cannot fit

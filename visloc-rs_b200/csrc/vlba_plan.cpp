@@ -1353,10 +1353,12 @@ size_t Plan::device_bytes() const {
   b += (size_t)num_var_cams * (4 + 4 + 4 + 4 + 36 * 4 + 6 * 4 * 6);
   b += tr_list.size() * 4 + (size_t)num_tile_rows * (4 + 4 + 16 * 8);
   b += chunk_point_begin.size() * (4 + 8 + 8 + 8);
-  // The team kernel's blocks, exchange words and tile lists.
+  // The team kernel's blocks, exchange words and tile lists (at most 16 blocks
+  // where the cluster kernels solve unless the device places none of 16 blocks).
   for (size_t p = 0; p + 1 < prob_tr_begin.size(); ++p) {
     const size_t R = prob_tr_begin[p + 1] - prob_tr_begin[p];
-    b += 64 + (R > kSmallPcgRows ? 148 * 576 + 384 * R + 8 * (R + 148) * std::min<size_t>(R, 192) : 0);
+    const size_t blocks = R > kSmallPcgRows ? 148 : R > 4 ? 16 : 0;
+    b += 64 + (blocks ? blocks * 576 + 384 * R + 8 * (R + blocks) * std::min<size_t>(R, 192) : 0);
   }
   b += cameras.size() * sizeof(DevCamera);
   return b;

@@ -211,6 +211,7 @@ struct Context {
   uint32_t flags = 0;  // flags of the uploaded config
   size_t l2_bytes = 0;
   double l2_fraction = 0.5;  // share of the L2 that keeps S resident in PCG
+  uint32_t small_rows = kSmallPcgRows;     // tile rows up to which the cluster kernels solve
   std::vector<uint32_t> team_round_begin;  // Dev::team_round_begin
   int pcg_grid_hint = 0;     // blocks of the PCG launch (trace sizing)
   // the uploaded problems' sizes (for download)
@@ -499,9 +500,10 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
   std::vector<uint32_t> tile_begin(P.num_problems + 1, 0u), small;
   for (size_t t = 0; t < P.tile_ij.size(); ++t) ++tile_begin[P.tile_meta[4 * t + 3] + 1];
   for (uint32_t p = 0; p < P.num_problems; ++p) tile_begin[p + 1] += tile_begin[p];
+  const auto rows = [&](uint32_t p) { return P.prob_tr_begin[p + 1] - P.prob_tr_begin[p]; };
   for (int k = 0; k < kSmallPcgClasses; ++k) {
     for (uint32_t p = 0; p < P.num_problems; ++p)
-      if (small_pcg_class(P.prob_tr_begin[p + 1] - P.prob_tr_begin[p]) == k) small.push_back(p);
+      if (rows(p) <= c->small_rows && small_pcg_class(rows(p)) == k) small.push_back(p);
     d.small_off[k + 1] = (uint32_t)small.size();
   }
   d.prob_tile_begin = st.up(A, tile_begin);
@@ -509,11 +511,10 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
   // Then the problems that fit a team of blocks; the persistent kernel has
   // the rest.
   TeamPlan team = build_team_plan(P.prob_tr_begin.data(), P.num_problems, P.tile_ij, tile_begin,
-                                        (uint32_t)c->sm_count);
+                                  c->small_rows, (uint32_t)c->sm_count);
   std::vector<uint8_t> big(P.num_problems, 0);
   for (uint32_t p = 0; p < P.num_problems; ++p) {
-    big[p] = !team.in_team[p] &&
-             small_pcg_class(P.prob_tr_begin[p + 1] - P.prob_tr_begin[p]) < 0;
+    big[p] = !team.in_team[p] && rows(p) > c->small_rows;
     d.num_big += big[p];
   }
   d.prob_big = st.up(A, big);
@@ -1461,6 +1462,9 @@ Context* make_context(int device) {
   c->l2_bytes = (size_t)prop.l2CacheSize;
   c->pcg_grid_hint = 4 * prop.multiProcessorCount;
   if (const char* f = std::getenv("VLBA_L2_RESIDENT_FRACTION")) c->l2_fraction = std::atof(f);
+  // VLBA_MAX_CLUSTER: the largest thread-block cluster this context uses (16).
+  const char* cl = std::getenv("VLBA_MAX_CLUSTER");
+  c->small_rows = small_pcg_rows(cl ? (uint32_t)std::max(0, std::atoi(cl)) : 16u);
   VLBA_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   VLBA_CUDA(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
   VLBA_CUDA(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
