@@ -172,6 +172,27 @@ def test_launch_shapes_do_not_change_results(solver):
         assert a.final_cost == b.final_cost
 
 
+def test_launch_shapes_are_kept_for_the_persistent_kernel_alone(solver, monkeypatch, capfd):
+    """576 and 584 densely coupled cameras fall into the same size buckets; a
+    team solves the first, the persistent kernel the second.  A shape measured
+    where that kernel does not run says nothing and is not kept for it."""
+    monkeypatch.setenv("VLBA_TRACE_UPLOAD", "1")
+    team, big = (synth.ring_problem(n + 2, 40 * n, seed=n) for n in (576, 584))
+    c = cfg(autotune=True, max_iterations=1)
+
+    def shapes(p):
+        st, _ = solver.optimize(p.copy(), c)
+        assert st == _abi.OK, solver.last_error()
+        return [s.split()[3].rstrip(",") for s in capfd.readouterr().err.splitlines()
+                if s.startswith("vlba launch shape:")]
+
+    capfd.readouterr()
+    assert shapes(team) == []
+    assert shapes(big) == ["measured"]
+    assert shapes(big) == ["cached"]
+    assert shapes(team) == []
+
+
 def test_observation_order_does_not_change_the_solve(solver):
     """Observations listed by landmark skip the plan's counting sort (its
     stable result is then the identity); listed in another order they go

@@ -283,10 +283,12 @@ uint32_t l2_tiles(const Context* c, double frac) {
 // shape for the process.  The tile size and the assembly's lane count set
 // summation orders, so they are not tuned: a problem must solve the same
 // alone and in any batch.
+// The shape is the persistent kernel's: an upload it solves nothing of takes
+// no part in the cache.
 struct ShapeKey {
-  uint32_t tiles, rows, problems;
+  uint32_t tiles, rows, problems, big;
   bool operator<(const ShapeKey& o) const {
-    return std::tie(tiles, rows, problems) < std::tie(o.tiles, o.rows, o.problems);
+    return std::tie(tiles, rows, problems, big) < std::tie(o.tiles, o.rows, o.problems, o.big);
   }
 };
 struct LaunchShape {
@@ -306,9 +308,16 @@ uint32_t log2_bucket(uint64_t v) {
   return b;
 }
 
-ShapeKey shape_key(const Plan& P) {
+// VLBA_TRACE_UPLOAD: the launch shape that was found or measured, to stderr.
+void trace_shape(const char* how, int grid, double l2_fraction) {
+  if (std::getenv("VLBA_TRACE_UPLOAD"))
+    std::fprintf(stderr, "vlba launch shape: %s, %d blocks, L2 share %.1f\n", how, grid, l2_fraction);
+}
+
+ShapeKey shape_key(const Context* c) {
+  const Plan& P = c->plan;
   return ShapeKey{log2_bucket(P.tile_ij.size()), log2_bucket(P.num_tile_rows),
-                  log2_bucket(P.num_problems)};
+                  log2_bucket(P.num_problems), log2_bucket(c->dev.num_big)};
 }
 
 int pcg_grid_max(const Context* c) {
@@ -707,14 +716,16 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
                      " tile rows per PCG block");
   if (P.num_tile_rows && c->pcg_grid <= 0)
     throw Status(VLBA_ERR_CUDA, "the PCG kernel cannot be made co-resident on this device");
-  // A launch shape tuned earlier for a system of this shape.
-  c->tuned = false;
-  {
+  // A launch shape tuned earlier for a system of this shape (none to choose
+  // where the persistent kernel solves nothing).
+  c->tuned = d.num_big == 0;
+  if (!c->tuned) {
     std::lock_guard<std::mutex> lock(g_tune_mu);
-    auto it = g_tune_cache.find(shape_key(P));
+    auto it = g_tune_cache.find(shape_key(c));
     if (it != g_tune_cache.end()) {
       apply_shape(c, it->second);
       c->tuned = true;
+      trace_shape("cached", c->pcg_grid, it->second.l2_fraction);
     }
   }
   if (c->dev.trace && c->pcg_grid > c->pcg_grid_hint) c->dev.trace = nullptr;  // sized for fewer blocks
@@ -1015,7 +1026,8 @@ RunStats run_lm(Context* c, bool profile, PhaseTimes* pt) {
 }
 
 // Times kIters PCG iterations (tolerance 0) on the system assembled at the
-// uploaded initial state for each candidate shape; keeps the fastest.
+// uploaded initial state for each candidate shape; keeps the fastest (the
+// default shape, timed alone, where the persistent kernel solves nothing).
 LaunchShape autotune(Context* c) {
   constexpr uint32_t kIters = 16;
   Dev& d = c->dev;
@@ -1043,14 +1055,19 @@ LaunchShape autotune(Context* c) {
   check_launch(launch_cam_diag(d, s), "camera blocks");
   const int gmax = pcg_grid_max(c), gmin = std::max(1, pcg_grid_min(c));
   std::vector<int> grids;
+  std::vector<double> fractions = {0.5, 0.0, 0.9};
+  if (!d.num_big) {
+    grids = {best.pcg_grid};
+    fractions = {best.l2_fraction};
+  }
   for (double f : {1.0, 0.75, 0.5, 0.375, 0.25, 0.125}) {
-    if (!d.num_big && !grids.empty()) break;  // the shape is the persistent kernel's
+    if (!d.num_big) break;
     const int g = std::max(gmin, (int)(f * gmax));
     if (std::find(grids.begin(), grids.end(), g) == grids.end()) grids.push_back(g);
   }
   double best_ms = 1e30;
   for (int g : grids)
-    for (double frac : {0.5, 0.0, 0.9}) {
+    for (double frac : fractions) {
       LaunchShape sh;
       sh.pcg_grid = g;
       sh.l2_fraction = frac;
@@ -1076,9 +1093,10 @@ LaunchShape autotune(Context* c) {
   VLBA_CUDA(cudaStreamSynchronize(s));
   best.pcg_iteration_us = 1e3 * best_ms / kIters;
   apply_shape(c, best);
-  {
+  if (d.num_big) {
     std::lock_guard<std::mutex> lock(g_tune_mu);
-    g_tune_cache[shape_key(P)] = best;
+    g_tune_cache[shape_key(c)] = best;
+    trace_shape("measured", c->pcg_grid, best.l2_fraction);
   }
   c->tuned = true;
   return best;
@@ -2932,7 +2950,7 @@ int visloc_ba_cuda_autotune(void* ctx, vlba_launch_shape* chosen) {
     vlba::set_device(c);
     {  // a new measurement, not the cached shape
       std::lock_guard<std::mutex> lock(vlba::g_tune_mu);
-      vlba::g_tune_cache.erase(vlba::shape_key(c->plan));
+      vlba::g_tune_cache.erase(vlba::shape_key(c));
     }
     const vlba::LaunchShape sh = vlba::autotune(c);
     if (chosen) {
