@@ -272,3 +272,19 @@ def test_accelerator_declines_intrinsics_refinement(flag):
     assert {k: p.world_to_camera for k, p in ba.poses.items()} == before
     res = acc.optimize(ba, BaConfig())
     assert res is not None and res.final_cost < 1e-12
+
+
+@pytest.mark.parametrize("cameras,points,seed,bound", [(20, 4000, 6, 4e-8), (50, 5000, 3, 7.9e-8)])
+def test_lanes_of_a_block_are_summed_without_loss(solver, cameras, points, seed, bound):
+    """Off-diagonal blocks summed on a warp each, against FP64.  What cannot be
+    avoided is the rounding of the terms and of the result to FP32 (2.4e-8
+    each for a random mantissa); 32 lanes' sums added in plain FP32 on top of
+    it gave 4.8e-8 and 8.2e-8 here, four lanes 4.3e-8 and 8.1e-8."""
+    p = synth.ring_problem(cameras, points, seed=seed)
+    cfg = BaConfig(robust_kernel=RobustKernel.huber(1.0))
+    S, _ = solver.reduced_system(p, cfg, 1e-3)
+    st, ref, _, _, _ = oracle.reduced_system(p, 1e-3, cfg, step=False)
+    assert st == _abi.OK
+    n = S.shape[0] // 6
+    off = np.kron(1.0 - np.eye(n), np.ones((6, 6)))
+    assert np.linalg.norm((S - ref) * off) <= bound * np.linalg.norm(ref * off)

@@ -419,6 +419,31 @@ __device__ __forceinline__ void point_inverse64(const Dev& d, uint32_t l, double
   v[2] = c[8];
 }
 
+// Sums of v[0..N) over the lanes that differ in bits OFF to 1, by a reduce-scatter:
+// the lanes with the bit clear keep the first half of the sums (rounded up), the
+// others the rest.  Returns this lane's first sum and their count, at the front
+// of v (at most two of 36 over all five bits).
+template <int N, int OFF>
+__device__ __forceinline__ uint2 scatter_sums(double* v, uint32_t lane, uint32_t first,
+                                              uint32_t count) {
+  constexpr int kHalf = (N + 1) / 2;
+  const bool upper = lane & (uint32_t)OFF;
+#pragma unroll
+  for (int e = 0; e < kHalf; ++e) {
+    const double hi = e + kHalf < N ? v[e + kHalf] : 0.0;
+    const double keep = upper ? hi : v[e], send = upper ? v[e] : hi;
+    v[e] = keep + __shfl_xor_sync(0xffffffffu, send, OFF);
+  }
+  if (upper) {
+    first += kHalf;
+    count = count > (uint32_t)kHalf ? count - kHalf : 0u;
+  } else {
+    count = min(count, (uint32_t)kHalf);
+  }
+  if constexpr (OFF > 1) return scatter_sums<kHalf, OFF / 2>(v, lane, first, count);
+  return make_uint2(first, count);
+}
+
 // ------------------------------------------------- off-diagonal Schur blocks
 // One group of G lanes per camera pair (i, j), i > j: lanes stride the pair's
 // points in order, each accumulating -B^T H_i H^-1 H_j B with compensated
@@ -435,7 +460,13 @@ __device__ __forceinline__ void point_inverse64(const Dev& d, uint32_t l, double
 // a warp then loop about as many times (lane-pass efficiency 0.82 -> 0.99 on
 // ring-4m) while the blocks running at one time stay those of nearby rows.
 // LONG: the blocks of the long list (long_block_terms) on G lanes each;
-// otherwise the other blocks in the length-sorted order.
+// otherwise the other blocks in the length-sorted order.  A long block's lanes
+// are added in FP64 with what their compensation holds: five plain FP32
+// additions in place of two lost more than four lanes do (off-diagonal blocks of
+// an 18-camera ring against FP64: 4 lanes 4.33e-8, 32 lanes added plainly
+// 4.79e-8, in FP64 3.25e-8).  The scatter takes 19 FP64 exchanges a lane after
+// the first 18 where the butterfly took 180 of FP32: a 20-keyframe window 14.6 ->
+// 13.9 us, 48 windows 155 -> 146.
 template <int G, bool LONG>
 __global__ void __launch_bounds__(256, 2) k_offdiag(Dev d) {
   constexpr int kPerWarp = 32 / G;
@@ -510,16 +541,36 @@ __global__ void __launch_bounds__(256, 2) k_offdiag(Dev d) {
         }
       }
     }
+    if constexpr (LONG) {
+      // The first step of the scatter as the sums widen.
+      const bool upper = lane & 16u;
+      double v[18];
 #pragma unroll
-    for (int off = G / 2; off > 0; off >>= 1)
+      for (int e = 0; e < 18; ++e) {
+        const double lo = (double)acc[e] - (double)cmp[e];
+        const double hi = (double)acc[e + 18] - (double)cmp[e + 18];
+        v[e] = (upper ? hi : lo) + __shfl_xor_sync(0xffffffffu, upper ? lo : hi, 16);
+      }
+      const uint2 mine = scatter_sums<18, 8>(v, lane, upper ? 18u : 0u, 18u);
 #pragma unroll
-      for (int e = 0; e < 36; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], off, G);
-    if (valid) {
+      for (uint32_t i = 0; i < 2; ++i) {
+        const uint32_t e = mine.x + i;
+        if (!valid || i >= mine.y) continue;
+        d.tiles[dst.x + e] = (float)v[i];
+        if (dst.y != kNone) d.tiles[dst.y + (e % 6) * 6 + e / 6] = (float)v[i];
+      }
+    } else {
 #pragma unroll
-      for (int e = 0; e < 36; ++e) {
-        if ((uint32_t)(e % G) == lane) {
-          d.tiles[dst.x + e] = acc[e];
-          if (dst.y != kNone) d.tiles[dst.y + (e % 6) * 6 + e / 6] = acc[e];
+      for (int off = G / 2; off > 0; off >>= 1)
+#pragma unroll
+        for (int e = 0; e < 36; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], off, G);
+      if (valid) {
+#pragma unroll
+        for (int e = 0; e < 36; ++e) {
+          if ((uint32_t)(e % G) == lane) {
+            d.tiles[dst.x + e] = acc[e];
+            if (dst.y != kNone) d.tiles[dst.y + (e % 6) * 6 + e / 6] = acc[e];
+          }
         }
       }
     }
