@@ -313,16 +313,6 @@ __device__ __forceinline__ unsigned long long now_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-
-// 1 / v for a positive normal v, to about two units in the last place: the
-// hardware's approximation and two Newton steps, a third of the latency of
-// the divide (the PCG's scalar chain).
-__device__ __forceinline__ double inverse64(double v) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
-  y = fma(y, fma(-v, y, 1.0), y);
-  return fma(y, fma(-v, y, 1.0), y);
-}
 #endif
 
 }  // namespace vlba

@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
   if (rr > 0.0 && rz > 0.0 && cap != 0u) {
     float beta = 0.0f;
     for (;;) {
-      const double inv_rz = inverse64(rz);
+      const double inv_rz = 1.0 / rz;  // for beta, off the chain of the sums
       float acc[N][6];
 #pragma unroll
       for (int u = 0; u < N; ++u)
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
         status = 2;  // non-positive curvature: x unchanged
         break;
       }
-      const float alpha = (float)(rz * inverse64(pq));
+      const float alpha = (float)(rz / pq);
       x = x + alpha * po;
       r = r - alpha * qa;
       precondition();

@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pcg_team(Dev d, uint32_t fi
   if (ok && rr > 0.0 && rz > 0.0 && cap != 0u) {
     float beta = 0.0f;
     for (;;) {
-      const double inv_rz = inverse64(rz);
+      const double inv_rz = 1.0 / rz;  // for beta, off the chain of the sums
       for (uint32_t e = 2u * tid; e < L; e += 2u * kTeamThreads) {
         const float2 zv = *reinterpret_cast<const float2*>(z_in + e);
         float2 pv = *reinterpret_cast<const float2*>(p + e);
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pcg_team(Dev d, uint32_t fi
         status = 2;  // non-positive curvature: x unchanged
         break;
       }
-      const float alpha = (float)(rz * inverse64(pq));
+      const float alpha = (float)(rz / pq);
       x = x + alpha * po;
       r = r - alpha * qa;
       exchange_z();
