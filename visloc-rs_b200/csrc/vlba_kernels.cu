@@ -1613,6 +1613,9 @@ __global__ void __launch_bounds__(Pcg::kThreads, 1) k_pcg(Dev d) {
   constexpr int NW = C::kWarps;
   extern __shared__ __align__(128) unsigned char smem[];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  // Every problem done (the iteration that the host had issued ahead): the same
+  // for every block, as the count falls only after the first grid barrier.
+  if (*(volatile unsigned int*)(d.barrier + 2) == 0u) return;
   // Per-warp region: kStages tile buffers, then the warp's p segments.
   unsigned char* wbase = smem + (size_t)warp * C::kWarpBytes;
   float* const ring = reinterpret_cast<float*>(wbase);
