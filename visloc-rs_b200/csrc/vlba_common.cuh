@@ -181,7 +181,7 @@ struct Dev {
   unsigned long long* team_z;      // (exchange number, z), each block's on lines of its own
   unsigned long long* team_slots;  // [2 kLineWords team_slots_total] (number, half of a double)
   uint32_t* team_epoch;            // [num_problems] last exchange number used
-  const uint8_t* prob_big;         // [num_problems] 1: the persistent kernel's
+  const uint32_t* prob_big;        // [num_problems] 1: the persistent kernel's
   const uint32_t* pose_prob;         // [num_poses]
   const uint32_t* point_prob;        // [num_points]
   const uint32_t* slot_prob;         // [num_var_cams]

@@ -476,42 +476,45 @@ size_t team_smem(uint32_t nodes, uint32_t ncols) {
 
 }  // namespace
 
-// Blocks of one problem for a team of `size`; the most parts of a block (its
-// bytes in *smem), or 0 when a block would own or read too many cameras or not
-// fit its shared memory.  `near` lists each tile row's columns (both triangles),
-// ascending.
-static uint32_t split_team(const std::vector<std::vector<uint32_t>>& near, uint32_t size,
-                           std::vector<TeamCta>* out, std::vector<uint32_t>* cols, size_t* smem) {
-  const uint32_t R = (uint32_t)near.size(), nodes = 8 * R;
-  uint32_t worst = 0;
-  std::vector<uint32_t> u;
+namespace {
+// The tile columns of each tile row (both triangles), a bit each.
+struct Near {
+  uint32_t rows, words;
+  std::vector<uint64_t> bits;
+  explicit Near(uint32_t r) : rows(r), words((r + 63) / 64), bits((size_t)r * words) {}
+  void set(uint32_t i, uint32_t j) { bits[(size_t)i * words + j / 64] |= 1ull << (j % 64); }
+};
+}  // namespace
+
+// Blocks of one problem for a team of `size`, whose largest needs *smem bytes;
+// false when a block would own or read too many cameras, have more than
+// `most` parts or not fit its shared memory.
+static bool split_team(const Near& near, uint32_t size, uint32_t most, std::vector<TeamCta>* out,
+                       std::vector<uint32_t>* cols, size_t* smem) {
+  const uint32_t nodes = 8 * near.rows;
+  std::vector<uint64_t> u(near.words);
   for (uint32_t g = 0; g < size; ++g) {
     TeamCta T{};
     T.rank = g;
     T.size = size;
     T.node0 = (uint32_t)((uint64_t)nodes * g / size);
     T.node1 = (uint32_t)((uint64_t)nodes * (g + 1) / size);
-    if (T.node1 == T.node0 || T.node1 - T.node0 > kTeamMaxNodes) return 0;
-    u.clear();
-    for (uint32_t I = T.node0 / 8; I <= (T.node1 - 1) / 8; ++I) {
-      const size_t mid = u.size();
-      u.insert(u.end(), near[I].begin(), near[I].end());
-      std::inplace_merge(u.begin(), u.begin() + (long)mid, u.end());
-    }
-    u.erase(std::unique(u.begin(), u.end()), u.end());
-    T.ncols = (uint32_t)u.size();
-    if (T.ncols > kTeamMaxCols) return 0;
-    worst = std::max(worst, team_parts(T.node1 - T.node0, T.ncols));
+    if (T.node1 == T.node0 || T.node1 - T.node0 > kTeamMaxNodes) return false;
+    std::fill(u.begin(), u.end(), 0ull);
+    for (uint32_t I = T.node0 / 8; I <= (T.node1 - 1) / 8; ++I)
+      for (uint32_t w = 0; w < near.words; ++w) u[w] |= near.bits[(size_t)I * near.words + w];
+    for (uint64_t w : u) T.ncols += (uint32_t)__builtin_popcountll(w);
+    if (T.ncols > kTeamMaxCols || team_parts(T.node1 - T.node0, T.ncols) > most) return false;
     const size_t bytes = team_smem(T.node1 - T.node0, T.ncols);
-    if (bytes > kTeamMaxSmem) return 0;
+    if (bytes > kTeamMaxSmem) return false;
     *smem = std::max(*smem, bytes);
-    if (out) {
-      T.col_begin = (uint32_t)cols->size();
-      cols->insert(cols->end(), u.begin(), u.end());
-      out->push_back(T);
-    }
+    if (!out) continue;
+    T.col_begin = (uint32_t)cols->size();
+    for (uint32_t w = 0; w < near.words; ++w)
+      for (uint64_t b = u[w]; b; b &= b - 1) cols->push_back(64 * w + (uint32_t)__builtin_ctzll(b));
+    out->push_back(T);
   }
-  return worst;
+  return true;
 }
 
 TeamPlan build_team_plan(const uint32_t* prob_tr_begin, uint32_t num_problems,
@@ -530,28 +533,26 @@ TeamPlan build_team_plan(const uint32_t* prob_tr_begin, uint32_t num_problems,
     if (R <= small_rows) continue;
     const uint32_t most = kRegParts + kExtra;
     const uint64_t tiles = tile_begin[p + 1] - tile_begin[p];
-    if ((2 * tiles - R) * 8 / kSegTiles > (uint64_t)max_blocks * most) continue;  // cannot fit
-    std::vector<std::vector<uint32_t>> near(R);
+    // What cannot fit: the parts or the cameras of all blocks.
+    if ((2 * tiles - R) * 8 / kSegTiles > (uint64_t)max_blocks * most ||
+        8 * (uint64_t)R > (uint64_t)max_blocks * kTeamMaxNodes)
+      continue;
+    Near near(R);
     for (uint32_t t = tile_begin[p]; t < tile_begin[p + 1]; ++t) {
       const uint32_t I = (tile_ij[t] >> 16) - tr0, J = (tile_ij[t] & 0xFFFFu) - tr0;
-      near[I].push_back(J);
-      if (I != J) near[J].push_back(I);
+      near.set(I, J);
+      near.set(J, I);
     }
-    for (auto& v : near) std::sort(v.begin(), v.end());
     uint32_t size = 0;
     for (uint32_t s : {16u, 24u, 32u, 48u, 64u, 80u, 96u, 112u, 128u, 148u}) {
       s = std::min(s, max_blocks);
       size_t bytes = 0;
-      const uint32_t worst = split_team(near, s, nullptr, nullptr, &bytes);
-      if (worst && (worst <= kRegParts || (s == max_blocks && worst <= most))) {
-        size = s;
-        break;
-      }
-      if (s == max_blocks) break;
+      if (split_team(near, s, s == max_blocks ? most : kRegParts, nullptr, nullptr, &bytes)) size = s;
+      if (size || s == max_blocks) break;
     }
     if (!size) continue;
     const uint32_t first = (uint32_t)tp.cta.size();
-    split_team(near, size, &tp.cta, &tp.cols, &tp.smem);
+    split_team(near, size, most, &tp.cta, &tp.cols, &tp.smem);
     // The tile of each (tile row, column) the block reads.
     std::vector<uint32_t> id((size_t)R * R, kNone);
     for (uint32_t t = tile_begin[p]; t < tile_begin[p + 1]; ++t) {
@@ -568,9 +569,11 @@ TeamPlan build_team_plan(const uint32_t* prob_tr_begin, uint32_t num_problems,
       T.z_own = own_words;
       own_words += (6 * (T.node1 - T.node0) + kLineWords - 1) / kLineWords * kLineWords;
       T.ent_begin = (uint32_t)tp.ents.size();
-      for (uint32_t I = T.node0 / 8; I <= (T.node1 - 1) / 8; ++I)
-        for (uint32_t k = 0; k < T.ncols; ++k)
-          tp.ents.push_back(id[(size_t)I * R + tp.cols[T.col_begin + k]]);
+      const uint32_t I0 = T.node0 / 8, I1 = (T.node1 - 1) / 8 + 1;
+      tp.ents.resize(tp.ents.size() + (size_t)(I1 - I0) * T.ncols);
+      uint32_t* e = tp.ents.data() + T.ent_begin;
+      for (uint32_t I = I0; I < I1; ++I)
+        for (uint32_t k = 0; k < T.ncols; ++k) *e++ = id[(size_t)I * R + tp.cols[T.col_begin + k]];
     }
     tp.z_words += own_words;
     tp.in_team[p] = 1;

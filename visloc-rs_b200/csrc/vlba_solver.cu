@@ -515,18 +515,15 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
       if (rows(p) <= c->small_rows && small_pcg_class(rows(p)) == k) small.push_back(p);
     d.small_off[k + 1] = (uint32_t)small.size();
   }
-  d.prob_tile_begin = st.up(A, tile_begin);
-  d.small_list = st.up(A, small);
   // Then the problems that fit a team of blocks; the persistent kernel has
   // the rest.
   TeamPlan team = build_team_plan(P.prob_tr_begin.data(), P.num_problems, P.tile_ij, tile_begin,
                                   c->small_rows, (uint32_t)c->sm_count);
-  std::vector<uint8_t> big(P.num_problems, 0);
+  std::vector<uint32_t> big(P.num_problems, 0u);
   for (uint32_t p = 0; p < P.num_problems; ++p) {
     big[p] = !team.in_team[p] && rows(p) > c->small_rows;
     d.num_big += big[p];
   }
-  d.prob_big = st.up(A, big);
   std::vector<uint32_t> long_terms(P.num_problems, 0u);  // blocks, then the threshold
   if (P.num_problems == 1) {
     long_terms[0] = (uint32_t)P.blk_dst.size();
@@ -535,15 +532,34 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
     for (const PairIdx& b : P.blk_dst) ++long_terms[P.tile_meta[4 * (size_t)(b.a / tf) + 3]];
   }
   for (uint32_t& n : long_terms) n = long_block_terms(n);
-  d.prob_long_terms = st.up(A, long_terms);
+  // One copy for these and the teams' lists: a copy of its own costs each some
+  // 5 us of the call, on a small system more than it saves.
+  std::vector<uint32_t> lists;
+  const auto put = [&lists](const uint32_t* v, size_t n) {
+    const size_t at = (lists.size() + 3) / 4 * 4;
+    lists.resize(at);
+    lists.insert(lists.end(), v, v + n);
+    return at;
+  };
+  const size_t at_tile = put(tile_begin.data(), tile_begin.size()), at_small = put(small.data(), small.size()),
+               at_big = put(big.data(), big.size()), at_long = put(long_terms.data(), long_terms.size()),
+               at_cta = put(reinterpret_cast<const uint32_t*>(team.cta.data()),
+                            team.cta.size() * (sizeof(TeamCta) / 4)),
+               at_cols = put(team.cols.data(), team.cols.size()),
+               at_ents = put(team.ents.data(), team.ents.size());
+  const uint32_t* const dev_lists = st.up(A, lists);
+  d.prob_tile_begin = dev_lists + at_tile;
+  d.small_list = dev_lists + at_small;
+  d.prob_big = dev_lists + at_big;
+  d.prob_long_terms = dev_lists + at_long;
   c->team_round_begin = std::move(team.round_begin);
   d.team_rounds = c->team_round_begin.empty() ? 0u : (uint32_t)c->team_round_begin.size() - 1;
   d.team_round_begin = c->team_round_begin.data();
   d.team_smem = (uint32_t)team.smem;
   d.team_slots_total = (uint32_t)team.cta.size();
-  d.team_cta = st.up(A, team.cta);
-  d.team_cols = st.up(A, team.cols);
-  d.team_ents = st.up(A, team.ents);
+  d.team_cta = reinterpret_cast<const TeamCta*>(dev_lists + at_cta);
+  d.team_cols = dev_lists + at_cols;
+  d.team_ents = dev_lists + at_ents;
   if (d.team_rounds) {
     // Number 0 is no exchange's.
     d.team_z = A.alloc<unsigned long long>(team.z_words + 2 * kLineWords * team.cta.size());
@@ -784,12 +800,12 @@ void dump_trace(Context* c) {
   VLBA_CUDA(cudaMemcpyAsync(t.data(), d.trace, t.size() * 8, cudaMemcpyDeviceToHost, c->stream));
   std::vector<PcgState> pg(d.num_problems);
   std::vector<Ctrl> ctrl(d.num_problems);
-  std::vector<uint8_t> big(d.num_problems);
+  std::vector<uint32_t> big(d.num_problems);
   VLBA_CUDA(cudaMemcpyAsync(pg.data(), d.pcg, pg.size() * sizeof(PcgState), cudaMemcpyDeviceToHost,
                             c->stream));
   VLBA_CUDA(cudaMemcpyAsync(ctrl.data(), d.ctrl, ctrl.size() * sizeof(Ctrl), cudaMemcpyDeviceToHost,
                             c->stream));
-  VLBA_CUDA(cudaMemcpyAsync(big.data(), d.prob_big, big.size(), cudaMemcpyDeviceToHost, c->stream));
+  VLBA_CUDA(cudaMemcpyAsync(big.data(), d.prob_big, 4 * big.size(), cudaMemcpyDeviceToHost, c->stream));
   VLBA_CUDA(cudaStreamSynchronize(c->stream));
   // The launch ran as long as its slowest problem.
   uint32_t most = 0;
