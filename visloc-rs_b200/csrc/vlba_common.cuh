@@ -111,13 +111,21 @@ struct PcgState {
 // kLongLanes lanes instead of the plan's lane count (a block's summation order
 // then depends on its own length and its problem's block count only, the same
 // alone and in any batch).  Where a problem's blocks are too few to fill the
-// device at four lanes each, every block takes a warp: a lane's terms are a
-// serial chain of gathers, about 1.1 us apiece.  Measured on B200 (assembly of
-// the off-diagonal blocks, 1,024 throughout against this rule): 153 blocks of
-// 200 terms 58 -> 15 us; 48 windows in a batch 325 -> 152 us; 27,000 blocks of a
-// street 267 -> 168 us; 717,000 blocks of 39 terms keep four lanes.
+// device at four lanes each, a lane's terms are a serial chain of gathers, about
+// 1.1 us apiece, and every block takes a warp.  With more blocks a warp pays
+// where a block is much longer than the others (a street's neighbouring
+// cameras); where most are of one length (a ring) a second launch for some of
+// them costs more than it saves.  Measured on B200 (us for the assembly phase, a
+// threshold of 1,024 terms throughout against this rule; the lines at 4,096 and
+// 32,768 blocks lie where the two sides meet, the threshold between them where
+// no ring is slower): rings of 40 cameras and 60 points a camera 38 and 25, 90
+// (4,005 blocks) 34 and 35, 100 33 and 34 (39 with a warp for every block), 180
+// and 140 points 55 and 55 (74 at 64 terms); streets of 300 cameras 64 and 52,
+// 400 144 and 92 (76 at 64 terms), 850 (28,000 blocks) 161 and 131; past 32,768
+// blocks 1,400 cameras 209 at 1,024 terms, 209 at 256, 223 at 64; 2,800 cameras
+// 368, 391 and 427.
 inline __host__ __device__ uint32_t long_block_terms(uint32_t problem_blocks) {
-  return problem_blocks <= 4096u ? 1u : problem_blocks <= 32768u ? 64u : 1024u;
+  return problem_blocks <= 4096u ? 1u : problem_blocks <= 32768u ? 192u : 1024u;
 }
 constexpr int kLongLanes = 32;
 
