@@ -100,6 +100,23 @@ def test_per_problem_configs_and_matching_the_oracle(solver):
         assert np.abs(b.camera_centers() - ref.camera_centers()).max() <= 1e-5 * extent
 
 
+def test_large_batches_sum_their_costs_as_each_alone(solver):
+    """Enough chunks of points for several to share a block (at the edges of
+    64-point chunks and 256-point blocks): the same bits as alone."""
+    sizes = [63, 64, 65, 128, 191, 192, 193, 255, 256, 257, 320, 511, 512, 513, 700, 1000]
+    probs = [synth.stereo_window(6 + i % 5, sizes[i % len(sizes)], seed=100 + i) for i in range(300)]
+    c = cfg(max_iterations=3)
+    batch = [p.copy() for p in probs]
+    statuses, results = solver.batch_optimize(batch, c)
+    assert statuses == [_abi.OK] * len(probs)
+    for i in list(range(16)) + [100, 239]:
+        alone = probs[i].copy()
+        st, res = solver.optimize(alone, c)
+        assert st == _abi.OK
+        assert res.initial_cost == results[i].initial_cost and res.final_cost == results[i].final_cost
+        assert same_state(alone, batch[i])
+
+
 def test_invalid_problems_are_left_out(solver):
     good = synth.stereo_window(10, 500, seed=7)
     bad = synth.ring_problem(6, 50, seed=3)

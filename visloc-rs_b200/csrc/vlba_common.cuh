@@ -137,6 +137,9 @@ constexpr int kLongLanes = 32;
 constexpr uint32_t kSmallPcgRows = 16;
 constexpr int kSmallPcgClasses = 4;
 
+// Chunks that a block of k_cost takes at most.
+constexpr uint32_t kCostChunks = 4;
+
 constexpr uint32_t kLineWords = 16;  // 64-bit words of a 128-byte line
 
 // One block of a problem's team (vlba_pcg_team.cu).
@@ -174,6 +177,8 @@ struct Dev {
   const uint32_t* prob_tr_begin;     // tile rows [num_problems + 1]
   const uint32_t* prob_tile_begin;   // tiles [num_problems + 1]
   const uint32_t* prob_chunk_begin;  // point chunks [num_problems + 1]
+  uint32_t num_cost_groups;
+  const uint2* cost_group;           // (chunk, point) where each block of k_cost begins [num_cost_groups + 1]
   // The problems of the small PCG kernels by class (small_pcg_class), and how
   // many problems the persistent kernel solves.
   const uint32_t* small_list;

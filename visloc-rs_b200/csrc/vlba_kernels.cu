@@ -93,42 +93,45 @@ __device__ __forceinline__ void btkb(const T* K, T x, T y, T z, T* out) {
   }
 }
 
-// Fixed-order sums of cost and bad and the maxima of step and (TWO) step2 over
+// Fixed-order sum of a double over a warp, in every lane.
+__device__ __forceinline__ double warp_total(double v) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
+}
+
+// Fixed-order sums of cost and bad and the maxima of step and step2 over
 // a block of 256 threads, in thread 0: a butterfly within each warp, then the
-// warps in order.  `red` is free again once every thread has passed the
-// second barrier.
-struct CostReduction {
+// warps in order.
+struct DecideReduction {
   double cost[8], step[8], step2[8];
   unsigned long long bad[8];
 };
-template <bool TWO>
-__device__ __forceinline__ void reduce_cost(double& cost, unsigned long long& bad, double& step,
-                                            double& step2, CostReduction& red) {
+__device__ __forceinline__ void reduce_decide(double& cost, unsigned long long& bad, double& step,
+                                              double& step2, DecideReduction& red) {
+  cost = warp_total(cost);
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
-    cost += __shfl_xor_sync(0xffffffffu, cost, off);
     bad += __shfl_xor_sync(0xffffffffu, bad, off);
     step = fmax(step, __shfl_xor_sync(0xffffffffu, step, off));
-    if (TWO) step2 = fmax(step2, __shfl_xor_sync(0xffffffffu, step2, off));
+    step2 = fmax(step2, __shfl_xor_sync(0xffffffffu, step2, off));
   }
   const uint32_t warp = threadIdx.x >> 5;
   if ((threadIdx.x & 31u) == 0) {
     red.cost[warp] = cost;
     red.bad[warp] = bad;
     red.step[warp] = step;
-    if (TWO) red.step2[warp] = step2;
+    red.step2[warp] = step2;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x != 0) return;
 #pragma unroll
-    for (int w = 1; w < 8; ++w) {
-      cost += red.cost[w];
-      bad += red.bad[w];
-      step = fmax(step, red.step[w]);
-      if (TWO) step2 = fmax(step2, red.step2[w]);
-    }
+  for (int w = 1; w < 8; ++w) {
+    cost += red.cost[w];
+    bad += red.bad[w];
+    step = fmax(step, red.step[w]);
+    step2 = fmax(step2, red.step2[w]);
   }
-  __syncthreads();
 }
 
 // 32-byte vector load (read-only path) and store: one request per 32-byte
@@ -939,32 +942,40 @@ __global__ void __launch_bounds__(256) k_pose_update(Dev d) {
 }
 
 // ------------------------------------------------- back-substitution + cost
-// One block of 256 threads per chunk of (at most 256) points of one problem,
-// in two steps.  With TRIAL, first the landmark step
+// One block of 256 threads per group of chunks of one problem (at most
+// kCostChunks chunks and 256 points), in two steps.  With TRIAL, first the landmark step
 //   dl = -H^-1 (g + sum_o H_o (rho + omega x X))
 // of every variable point (W_o^T dc = H_o B dc) and the candidate point
-// X + dl: the chunk's observations (contiguous) each form their term
+// X + dl: the group's observations (contiguous) each form their term
 // H_o (rho + omega x X) on one thread, kObsStage per pass, into shared
 // memory, and each point's thread adds its own terms from there in
-// observation order.  Then one thread per observation of the chunk for the
-// cost at the candidate poses/points (the current state without TRIAL).
-// Sums in a fixed order per chunk.
+// observation order.  Then one thread per observation, chunk after chunk, for
+// the cost at the candidate poses/points (the current state without TRIAL).
+// A chunk's cost is summed in an order fixed by the chunk, however the chunks are
+// grouped: a chunk a block where that fills few SMs, chunks of small problems
+// four to a block in a large batch (Dev::cost_group), where a block's chain of
+// loads is what counts.  Measured on B200 (update phase of 512 windows of up to
+// 5,000 points: 374 us in chunks of 256, 467 in chunks of 64 a block each, 381
+// grouped; 16 windows 42, 34 and 34).  Five blocks to an SM: with 63 registers
+// instead of 48, four, 60 windows took 75 us instead of 67.
 template <bool TRIAL>
-__global__ void __launch_bounds__(256) k_cost(Dev d) {
-  __shared__ CostReduction red;
-  __shared__ double sX[3 * 256];                      // the chunk's (candidate) points
+__global__ void __launch_bounds__(256, 5) k_cost(Dev d) {
+  __shared__ double s_cost[kCostChunks][8], s_step[8];
+  __shared__ unsigned long long s_bad[8];
+  __shared__ double sX[3 * 256];                      // the group's (candidate) points
   __shared__ float sXf[TRIAL ? 3 * 256 : 1];          // the points as FP32 (pt_s)
   __shared__ double sC[TRIAL ? 3 * kObsStage : 1];    // staged observation terms
   __shared__ unsigned char sAct[TRIAL ? 256 : 1];     // point takes a step
-  for (uint32_t ch = blockIdx.x; ch < d.num_point_chunks; ch += gridDim.x) {
-    const uint32_t lo = d.chunk_point_begin[ch], hi = d.chunk_point_begin[ch + 1];
+  for (uint32_t g = blockIdx.x; g < d.num_cost_groups; g += gridDim.x) {
+    const uint2 at0 = d.cost_group[g], at1 = d.cost_group[g + 1];
+    const uint32_t ch0 = at0.x, ch1 = at1.x, lo = at0.y, hi = at1.y;
     const uint32_t P = d.num_problems == 1 ? 0u : d.point_prob[lo];
     const Ctrl& c = d.ctrl[P];
-    if (c.done) continue;  // uniform: a chunk lies inside one problem
+    if (c.done) continue;  // uniform: a group lies inside one problem
     const uint32_t cur = c.cur;
     const uint32_t pose_buf = TRIAL ? (cur ^ 1u) : cur;
     const LmParams& lp = d.params[P];
-    double cost = 0.0, step = 0.0;
+    double step = 0.0;
     unsigned long long bad = 0;
     const uint32_t l = lo + threadIdx.x;
     const bool mine = l < hi;
@@ -1056,47 +1067,76 @@ __global__ void __launch_bounds__(256) k_cost(Dev d) {
       for (int a = 0; a < 3; ++a) sX[3 * threadIdx.x + a] = X[a];
     }
     __syncthreads();
-    // The chunk's observations, one thread each (stride 256), at the points
+    // Each chunk's observations, one thread each (stride 256), at the points
     // just placed in shared memory.
-    const uint32_t o0 = d.pt_off[lo], o1 = d.pt_off[hi];
-    for (uint32_t k = o0 + threadIdx.x; k < o1; k += blockDim.x) {
-      const double* Xk = sX + 3 * (d.obs_point[k] - lo);
-      const DevCamera& cam = d.cameras[d.obs_cam[k]];
-      double rt[12];
-      load_rt(d.pose_rt[pose_buf] + 12 * (size_t)d.obs_pose[k], rt);
-      double xs[3], pred[2];
-      to_sensor(rt, cam, Xk, xs);
-      double ss;
-      const uint32_t kind = d.obs_kind ? d.obs_kind[k] : kObsMono;
-      if (kind != kObsMono) {
-        double r[4];
-        const int m = stereo_rows(kind, cam, d.cameras[d.obs_rcam[k]], d.obs_xy[k], d.obs_st[k], xs,
-                                  nullptr, r, nullptr);
-        if (!m) {
-          ++bad;
-          continue;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t o1 = d.pt_off[lo];
+    for (uint32_t ch = ch0; ch < ch1; ++ch) {
+      const uint32_t o0 = o1;
+      o1 = d.pt_off[ch + 1 == ch1 ? hi : d.chunk_point_begin[ch + 1]];
+      double cost = 0.0;
+      for (uint32_t k = o0 + threadIdx.x; k < o1; k += blockDim.x) {
+        const double* Xk = sX + 3 * (d.obs_point[k] - lo);
+        const DevCamera& cam = d.cameras[d.obs_cam[k]];
+        double rt[12];
+        load_rt(d.pose_rt[pose_buf] + 12 * (size_t)d.obs_pose[k], rt);
+        double xs[3], pred[2];
+        to_sensor(rt, cam, Xk, xs);
+        double ss;
+        const uint32_t kind = d.obs_kind ? d.obs_kind[k] : kObsMono;
+        if (kind != kObsMono) {
+          double r[4];
+          const int m = stereo_rows(kind, cam, d.cameras[d.obs_rcam[k]], d.obs_xy[k], d.obs_st[k], xs,
+                                    nullptr, r, nullptr);
+          if (!m) {
+            ++bad;
+            continue;
+          }
+          ss = 0.0;
+          for (int i = 0; i < m; ++i) ss += r[i] * r[i];
+        } else {
+          if (!(xs[2] > 0.0) || !camera_project(cam, xs, pred)) {
+            ++bad;
+            continue;
+          }
+          const double2 xy = d.obs_xy[k];
+          const double rx = pred[0] - xy.x, ry = pred[1] - xy.y;
+          ss = rx * rx + ry * ry;
         }
-        ss = 0.0;
-        for (int i = 0; i < m; ++i) ss += r[i] * r[i];
-      } else {
-        if (!(xs[2] > 0.0) || !camera_project(cam, xs, pred)) {
-          ++bad;
-          continue;
-        }
-        const double2 xy = d.obs_xy[k];
-        const double rx = pred[0] - xy.x, ry = pred[1] - xy.y;
-        ss = rx * rx + ry * ry;
+        const double rc = robust_cost(lp.robust_kernel, lp.robust_parameter, ss);
+        cost += d.obs_w ? d.obs_w[k] * rc : rc;  // w * rho(s) (problem.rs:497-560)
       }
-      const double rc = robust_cost(lp.robust_kernel, lp.robust_parameter, ss);
-      cost += d.obs_w ? d.obs_w[k] * rc : rc;  // w * rho(s) (problem.rs:497-560)
+      cost = warp_total(cost);
+      if (lane == 0) s_cost[ch - ch0][warp] = cost;
     }
-    double none = 0.0;
-    reduce_cost<false>(cost, bad, step, none, red);
-    if (threadIdx.x == 0) {
-      d.chunk_cost[ch] = cost;
-      d.chunk_bad[ch] = bad;
-      d.chunk_step[ch] = step;
+    // The counts and maxima of the group with its first chunk.
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      bad += __shfl_xor_sync(0xffffffffu, bad, off);
+      step = fmax(step, __shfl_xor_sync(0xffffffffu, step, off));
     }
+    if (lane == 0) {
+      s_bad[warp] = bad;
+      s_step[warp] = step;
+    }
+    __syncthreads();
+    if (threadIdx.x < ch1 - ch0) {
+      double total = s_cost[threadIdx.x][0], top = 0.0;
+      unsigned long long count = 0;
+#pragma unroll
+      for (int w = 1; w < 8; ++w) total += s_cost[threadIdx.x][w];
+      if (threadIdx.x == 0) {
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+          count += s_bad[w];
+          top = fmax(top, s_step[w]);
+        }
+      }
+      d.chunk_cost[ch0 + threadIdx.x] = total;
+      d.chunk_bad[ch0 + threadIdx.x] = count;
+      d.chunk_step[ch0 + threadIdx.x] = top;
+    }
+    __syncthreads();
   }
 }
 
@@ -1108,7 +1148,7 @@ __global__ void __launch_bounds__(256) k_cost(Dev d) {
 // A non-finite step is the reference's SingularSystem: lambda up, no step.
 template <bool INIT>
 __global__ void __launch_bounds__(256) k_decide(Dev d) {
-  __shared__ CostReduction red;
+  __shared__ DecideReduction red;
   const uint32_t P = blockIdx.x;
   if (P >= d.num_problems) return;
   if (P == 0 && threadIdx.x == 0) d.host_state[1] = *(volatile unsigned int*)d.error;
@@ -1133,7 +1173,7 @@ __global__ void __launch_bounds__(256) k_decide(Dev d) {
     for (uint32_t p = d.prob_pose_begin[P] + threadIdx.x; p < d.prob_pose_begin[P + 1];
          p += blockDim.x)
       pstep = fmax(pstep, d.pose_step[p]);
-  reduce_cost<true>(cost, bad, lstep, pstep, red);
+  reduce_decide(cost, bad, lstep, pstep, red);
   if (threadIdx.x != 0) return;
   if (INIT) {
     c.initial_cost = cost;
@@ -2410,7 +2450,7 @@ cudaError_t launch_pose_table(const Dev& d, cudaStream_t s) {
 }
 
 cudaError_t launch_cost(const Dev& d, bool trial, cudaStream_t s) {
-  const int g = grid1d((size_t)d.num_point_chunks * 256, 256, 148 * 16);
+  const int g = grid1d((size_t)d.num_cost_groups * 256, 256, 148 * 16);
   if (trial)
     k_cost<true><<<g, 256, 0, s>>>(d);
   else

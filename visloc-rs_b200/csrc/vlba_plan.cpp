@@ -856,7 +856,8 @@ void build_plan_serial(const vlba_problem* const* problems, const vlba_config* c
     // takes small ones, enough to reach most SMs, at most 256 points otherwise.
     // Measured on B200 (k_cost, 256 points a chunk against this rule): 2,000
     // points 29 -> 13 us, 5,000 29 -> 13, 48 problems of 200 to 5,000 in a
-    // batch 37 -> 40 (54 at 32 points, whose blocks cost more than they bring).
+    // batch 37 -> 40 (54 at 32 points, whose blocks cost more than they bring);
+    // a large batch takes several chunks to a block (cost_groups).
     const uint32_t chunk = nl <= 148u * 64u ? 64u : nl <= 148u * 128u ? 128u : 256u;
     for (uint32_t j0 = 0; j0 < nl; j0 += chunk)
       P.chunk_point_begin.push_back(point_base + std::min(nl, j0 + chunk));

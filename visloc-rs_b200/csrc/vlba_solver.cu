@@ -474,6 +474,28 @@ void check_launch(cudaError_t e, const char* what) {
   if (e != cudaSuccess) throw CudaError(e, what);
 }
 
+// (First chunk, first point) of each block of k_cost, and the end: the chunks of
+// a problem taken in its order, as many as 256 points hold if that leaves at
+// least `least` blocks, else one.
+std::vector<uint32_t> cost_groups(const Plan& P, uint32_t least) {
+  const auto& at = P.chunk_point_begin;
+  std::vector<uint32_t> out;
+  const auto build = [&](uint32_t most) {
+    out.clear();
+    for (uint32_t p = 0; p < P.num_problems; ++p)
+      for (uint32_t c = P.prob_chunk_begin[p], end = P.prob_chunk_begin[p + 1]; c < end;) {
+        out.insert(out.end(), {c, at[c]});
+        uint32_t n = 1;
+        while (n < most && c + n < end && at[c + n + 1] - at[c] <= 256) ++n;
+        c += n;
+      }
+    out.insert(out.end(), {(uint32_t)at.size() - 1, at.back()});
+  };
+  build(kCostChunks);
+  if (out.size() / 2 <= least) build(1);
+  return out;
+}
+
 // `before_kernels` (if set) runs before the first kernel that reads the
 // plan's arrays: the copies may start while the host still checks the plan.
 void upload_plan_once(Context* c, uint32_t max_records, const std::function<void()>& before_kernels) {
@@ -532,6 +554,13 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
     for (const PairIdx& b : P.blk_dst) ++long_terms[P.tile_meta[4 * (size_t)(b.a / tf) + 3]];
   }
   for (uint32_t& n : long_terms) n = long_block_terms(n);
+  // The groups of chunks that a block of k_cost takes: as many as 256 points
+  // hold where that still gives each SM three blocks (five fit).  Measured on
+  // B200 (update phase, a chunk a block and grouped): 24 windows of 200 to 5,000
+  // points, 250 groups, 44 and 47 us; 32 windows 52 and 58; 48 windows, 490
+  // groups, 65 and 65; 60 windows 75 and 67; 512 windows 467 and 376.
+  const std::vector<uint32_t> cost_group = cost_groups(P, 3u * (uint32_t)c->sm_count);
+  d.num_cost_groups = (uint32_t)cost_group.size() / 2 - 1;
   // One copy for these and the teams' lists: a copy of its own costs each some
   // 5 us of the call, on a small system more than it saves.
   std::vector<uint32_t> lists;
@@ -543,6 +572,7 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
   };
   const size_t at_tile = put(tile_begin.data(), tile_begin.size()), at_small = put(small.data(), small.size()),
                at_big = put(big.data(), big.size()), at_long = put(long_terms.data(), long_terms.size()),
+               at_cost = put(cost_group.data(), cost_group.size()),
                at_cta = put(reinterpret_cast<const uint32_t*>(team.cta.data()),
                             team.cta.size() * (sizeof(TeamCta) / 4)),
                at_cols = put(team.cols.data(), team.cols.size()),
@@ -551,6 +581,7 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
   d.prob_tile_begin = dev_lists + at_tile;
   d.small_list = dev_lists + at_small;
   d.prob_big = dev_lists + at_big;
+  d.cost_group = reinterpret_cast<const uint2*>(dev_lists + at_cost);
   d.prob_long_terms = dev_lists + at_long;
   c->team_round_begin = std::move(team.round_begin);
   d.team_rounds = c->team_round_begin.empty() ? 0u : (uint32_t)c->team_round_begin.size() - 1;
