@@ -189,6 +189,34 @@ def test_launch_shapes_do_not_change_results(solver):
         assert a.final_cost == b.final_cost
 
 
+def test_launch_shapes_do_not_change_results_of_the_persistent_kernel(solver):
+    """As above, on a batch whose second problem k_pcg solves (the shape is its
+    own: the others' kernels do not depend on it)."""
+    probs = [synth.stereo_window(20, 800, seed=2), synth.ring_problem(620, 24800, seed=7),
+             synth.ring_problem(150, 6000, seed=3)]
+    c = cfg(max_iterations=4, max_pcg_iterations=40)
+    outs = []
+    for blocks, l2 in ((0, 0.5), (17, 0.0), (40, 0.9), (148, 0.2)):
+        solver.batch_upload([p.copy() for p in probs], c)
+        solver.set_launch_shape(blocks, l2)
+        res = solver.batch_solve_uploaded()
+        out = [p.copy() for p in probs]
+        solver.batch_download(out)
+        outs.append((res, out))
+    solver.batch_upload([p.copy() for p in probs], c)
+    shape = solver.autotune()
+    assert shape["pcg_blocks"] >= 1 and shape["pcg_iteration_us"] > 0.0
+    res = solver.batch_solve_uploaded()
+    out = [p.copy() for p in probs]
+    solver.batch_download(out)
+    outs.append((res, out))
+    (r0, o0) = outs[0]
+    for r, o in outs[1:]:
+        for a, b, pa, pb in zip(r0, r, o0, o):
+            assert a.final_cost == b.final_cost
+            assert same_state(pa, pb)
+
+
 def test_launch_shapes_are_kept_for_the_persistent_kernel_alone(solver, monkeypatch, capfd):
     """576 and 584 densely coupled cameras fall into the same size buckets; a
     team solves the first, the persistent kernel the second.  A shape measured

@@ -1,7 +1,7 @@
 """The PCG kernels of reduced systems that stay on the chip at the sizes where
 one begins and ends, against the FP64 iteration they restate: the clusters
-(at most 16 tile rows, 128 cameras), the teams of blocks (up to about 450
-densely coupled cameras), and past them the persistent kernel."""
+(at most 16 tile rows, 128 cameras), the teams of blocks (up to 576 densely
+coupled cameras), and past them the persistent kernel."""
 
 from __future__ import annotations
 
@@ -86,7 +86,44 @@ def test_matches_the_fp64_iteration(solver, n, keep):
     assert np.array_equal(again, x)
 
 
-@pytest.mark.parametrize("n", [3, 20, 50, 100, 140, 480])
+def kernel_of(s, problem, monkeypatch, capfd):
+    """Which PCG kernel solves the problem: the persistent one alone fills the
+    phase trace, and only a team has waits for the probe to run out."""
+    with monkeypatch.context() as m:
+        m.setenv("VLBA_TRACE_PCG", "1")
+        capfd.readouterr()
+        st, _ = s.optimize(problem.copy(), BaConfig(max_iterations=1, max_pcg_iterations=3))
+        assert st == 0
+        if "vlba pcg trace:" in capfd.readouterr().err:
+            return "persistent"
+    s.wait_probe(1.0)
+    return "team" if "a bounded device wait" in s.last_error() else "cluster"
+
+
+@pytest.mark.parametrize("cameras,kernel", [(128, "cluster"), (129, "team"), (576, "team"),
+                                            (577, "persistent")])
+def test_the_kernel_of_a_dense_system_follows_its_size(solver, cameras, kernel, monkeypatch, capfd):
+    p = synth.ring_problem(cameras + 2, 40 * cameras, seed=cameras)  # two cameras are fixed
+    assert kernel_of(solver, p, monkeypatch, capfd) == kernel
+
+
+@pytest.mark.parametrize("n", [513, 520, 569, 576, 577, 584, 600])
+def test_dense_systems_at_the_limit_of_the_teams(solver, n):
+    """The largest layouts of a team (576 nodes: 36 parts a block, 20 of them in
+    shared memory) and the first sizes of the persistent kernel."""
+    diag, edges, off, rhs = system(n, 1.0, n)
+    S = dense(diag, edges, off)
+    x3, it3, _ = solver.reduced_solve(diag, edges, off, rhs, 0.0, 3)
+    ref3, _ = pcg64(S, diag, rhs, -1.0, 3)
+    assert it3 == 3
+    assert np.linalg.norm(x3.reshape(-1) - ref3) <= 1e-5 * np.linalg.norm(ref3)
+    x, it, rr = solver.reduced_solve(diag, edges, off, rhs, 1e-5, 300)
+    _, it_ref = pcg64(S, diag, rhs, 1e-5, 300)
+    assert abs(it - it_ref) <= 1 and rr <= 1e-5
+    assert np.linalg.norm(S @ x.reshape(-1) - rhs.reshape(-1)) <= 2e-5 * np.linalg.norm(rhs)
+
+
+@pytest.mark.parametrize("n", [3, 20, 50, 100, 140, 480, 600])
 def test_stopping_rules(solver, n):
     """Zero right-hand side, iteration cap 0 and 1, non-positive curvature
     (x stays at the last iterate) and NaN: as the persistent kernel."""
@@ -120,10 +157,11 @@ def test_a_negative_tolerance_is_never_met(solver, cameras):
     assert zero[2] == 9 and np.array_equal(never[0], zero[0])
 
 
-@pytest.mark.parametrize("band", [2, 9, 40])
+@pytest.mark.parametrize("band", [2, 9, 40, 60, 120])
 def test_banded_team(solver, band):
     """A long chain (1,400 nodes, more tile rows than blocks at the widest
-    team): each block reads its own stretch of columns."""
+    team): each block reads its own stretch of columns.  The widest band fits
+    no team."""
     n = 1400
     rng = np.random.default_rng(band)
     a = np.repeat(np.arange(n), band)
@@ -142,12 +180,17 @@ def test_banded_team(solver, band):
     assert np.linalg.norm(x.reshape(-1) - ref) <= 1e-5 * np.linalg.norm(ref)
 
 
-def test_teams_solve_the_same_alone_and_in_a_batch(solver):
-    """Problems of every PCG kernel in one batch (teams in two rounds): the
-    bits of each solved alone."""
+@pytest.mark.parametrize("big", [False, True])
+def test_teams_solve_the_same_alone_and_in_a_batch(solver, big):
+    """Problems of the cluster and team kernels, and with `big` of the
+    persistent one, in one batch (teams in two rounds): the bits of each
+    solved alone."""
     probs = [synth.ring_problem(140, 6000, seed=1), synth.stereo_window(20, 800, seed=2),
              synth.ring_problem(200, 8000, seed=3), synth.ring_problem(300, 20000, seed=4),
              synth.street_loop(500, 20000, seed=5), synth.ring_problem(100, 4000, seed=6)]
+    if big:
+        probs[1:1] = [synth.ring_problem(610, 24400, seed=7)]
+        probs.append(synth.ring_problem(700, 21000, seed=8))
     cfg = BaConfig(max_iterations=4, robust_kernel=RobustKernel.huber(1.0), max_pcg_iterations=60,
                    pcg_relative_tolerance=1e-6)
     alone = [p.copy() for p in probs]
@@ -164,6 +207,25 @@ def test_teams_solve_the_same_alone_and_in_a_batch(solver):
         for a, b, c, r in zip(alone, batch, costs, results):
             assert r.final_cost == c
             assert np.array_equal(a.pose_q, b.pose_q) and np.array_equal(a.landmarks, b.landmarks)
+
+
+def test_finished_problems_of_the_persistent_kernel_stay_out(solver):
+    """Iteration caps apart: each kernel's problems end at their own iteration
+    while the others go on, in either order."""
+    probs = [synth.ring_problem(610, 24400, seed=7), synth.ring_problem(40, 2000, seed=2),
+             synth.ring_problem(620, 24800, seed=9), synth.ring_problem(200, 8000, seed=3)]
+    for caps in ((1, 4, 3, 2), (4, 1, 2, 3)):
+        cfgs = [BaConfig(max_iterations=m, robust_kernel=RobustKernel.huber(1.0),
+                         max_pcg_iterations=40, pcg_relative_tolerance=1e-6) for m in caps]
+        batch = [p.copy() for p in probs]
+        statuses, results = solver.batch_optimize(batch, cfgs)
+        assert statuses == [0] * len(probs)
+        for p, b, c, r in zip(probs, batch, cfgs, results):
+            alone = p.copy()
+            st, res = solver.optimize(alone, c)
+            assert st == 0 and res.final_cost == r.final_cost
+            assert [i.pcg_iterations for i in res.iterations] == [i.pcg_iterations for i in r.iterations]
+            assert np.array_equal(alone.pose_q, b.pose_q) and np.array_equal(alone.landmarks, b.landmarks)
 
 
 def test_each_round_of_teams_is_a_launch(solver):
