@@ -326,6 +326,36 @@ __device__ __forceinline__ unsigned long long now_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
+
+// Sum over a warp in a fixed order, in every lane.
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
+}
+
+// Sums over a warp of each lane's six row products of S p: a reduce-scatter (lane
+// bit 4 keeps three of the six rows, bit 3 two or one of those), then a
+// butterfly.  Rows 0 and 2 (3 and 5 where bit 4 is set) in u of the lanes whose
+// bit 3 is clear and set, row 1 (4) in v of the lanes whose bit 3 is clear.
+__device__ __forceinline__ void row_sums(const float (&acc)[6], uint32_t lane, float& u, float& v) {
+  const bool b4 = (lane >> 4) & 1u, b3 = (lane >> 3) & 1u;
+  float h[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const float keep = b4 ? acc[q + 3] : acc[q], send = b4 ? acc[q] : acc[q + 3];
+    h[q] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+  }
+  const float g0 = __shfl_xor_sync(0xffffffffu, b3 ? h[0] : h[2], 8);
+  const float g1 = __shfl_xor_sync(0xffffffffu, h[1], 8);
+  u = b3 ? h[2] + g0 : h[0] + g0;
+  v = h[1] + g1;
+#pragma unroll
+  for (int off = 4; off > 0; off >>= 1) {
+    u += __shfl_xor_sync(0xffffffffu, u, off);
+    v += __shfl_xor_sync(0xffffffffu, v, off);
+  }
+}
 #endif
 
 }  // namespace vlba

@@ -93,13 +93,6 @@ __device__ __forceinline__ void btkb(const T* K, T x, T y, T z, T* out) {
   }
 }
 
-// Fixed-order sum of a double over a warp, in every lane.
-__device__ __forceinline__ double warp_total(double v) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  return v;
-}
-
 // Fixed-order sums of cost and bad and the maxima of step and step2 over
 // a block of 256 threads, in thread 0: a butterfly within each warp, then the
 // warps in order.
@@ -109,7 +102,7 @@ struct DecideReduction {
 };
 __device__ __forceinline__ void reduce_decide(double& cost, unsigned long long& bad, double& step,
                                               double& step2, DecideReduction& red) {
-  cost = warp_total(cost);
+  cost = warp_sum(cost);
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
     bad += __shfl_xor_sync(0xffffffffu, bad, off);
@@ -1106,7 +1099,7 @@ __global__ void __launch_bounds__(256, 5) k_cost(Dev d) {
         const double rc = robust_cost(lp.robust_kernel, lp.robust_parameter, ss);
         cost += d.obs_w ? d.obs_w[k] * rc : rc;  // w * rho(s) (problem.rs:497-560)
       }
-      cost = warp_total(cost);
+      cost = warp_sum(cost);
       if (lane == 0) s_cost[ch - ch0][warp] = cost;
     }
     // The counts and maxima of the group with its first chunk.
@@ -1456,12 +1449,6 @@ __device__ __forceinline__ int mod3(int k) { return ((k % 3) + 3) % 3; }
 constexpr int kDotRz = 0, kDotRr = 3, kDotPq = 6, kDotB2 = 8;
 __device__ __forceinline__ double* dot_at(const Dev& d, int slot, uint32_t tr) {
   return d.dots + (size_t)slot * d.num_tile_rows + tr;
-}
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  return v;
 }
 
 // Sums of a problem's tile-row dots (rz(k-1), rz(k-2), rr(k-1), pq(k-1), b2)

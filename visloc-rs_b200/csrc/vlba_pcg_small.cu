@@ -42,11 +42,6 @@
 namespace vlba {
 namespace {
 
-__device__ __forceinline__ double warp_sum_all(double v) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  return v;
-}
 // Sum over lanes 0-7 (lanes 6 and 7 hold zero), in lane 0 and its group.
 __device__ __forceinline__ double group_sum(double v) {
 #pragma unroll
@@ -203,7 +198,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
     for (int n = kLane; n > 1; n = (n + 1) / 2)
 #pragma unroll
       for (int i = 0; i < n / 2; ++i) v[i] += v[n - 1 - i];
-    return warp_sum_all(v[0]);
+    return warp_sum(v[0]);
   };
   // The sums every thread of the block needs, each by one warp: with all
   // sixteen summing for themselves the shuffle unit was the bound.
@@ -247,29 +242,14 @@ __global__ void __launch_bounds__(32 * W, 1) k_pcg_small(Dev d, const uint32_t* 
           for (int q = 0; q < 6; ++q) acc[u][q] = __fmaf_rn(S[u][q][j], p[j], acc[u][q]);
       }
       po = __fmaf_rn(beta, po, z);
-      // Row sums over the lanes: a reduce-scatter (bit 4 keeps three of the
-      // six rows, bit 3 two or one of those), then a butterfly; then row a
-      // back to its lane.
-      const bool b4 = (lane >> 4) & 1u, b3 = (lane >> 3) & 1u;
+      // The row sums over the lanes, row a back to its lane.
       const uint32_t part = a >= 3u ? a - 3u : a;
       const uint32_t src = (a >= 3u ? 16u : 0u) + (part == 2u ? 8u : 0u);
       float qa = 0.0f;
 #pragma unroll
       for (int w = 0; w < N; ++w) {
-        float h[3];
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          const float keep = b4 ? acc[w][q + 3] : acc[w][q], send = b4 ? acc[w][q] : acc[w][q + 3];
-          h[q] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-        }
-        const float g0 = __shfl_xor_sync(0xffffffffu, b3 ? h[0] : h[2], 8);
-        const float g1 = __shfl_xor_sync(0xffffffffu, h[1], 8);
-        float u = b3 ? h[2] + g0 : h[0] + g0, v = h[1] + g1;  // v: rows 1 and 4, where b3 is 0
-#pragma unroll
-        for (int off = 4; off > 0; off >>= 1) {
-          u += __shfl_xor_sync(0xffffffffu, u, off);
-          v += __shfl_xor_sync(0xffffffffu, v, off);
-        }
+        float u, v;
+        row_sums(acc[w], lane, u, v);
         const float qu = __shfl_sync(0xffffffffu, u, src), qv = __shfl_sync(0xffffffffu, v, src);
         if (sub == (uint32_t)w) qa = part == 1u ? qv : qu;
       }

@@ -67,11 +67,6 @@ constexpr uint32_t kExtra = 22;                       // parts kept in shared me
 // this one was about to launch with.
 constexpr size_t kTeamMaxSmem = (227 - 1) * 1024;
 
-__device__ __forceinline__ double warp_sum_t(double v) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  return v;
-}
 __device__ __forceinline__ void put_word(unsigned long long* a, uint32_t value, uint32_t epoch) {
   const unsigned long long w = ((unsigned long long)epoch << 32) | value;
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(a), "l"(w) : "memory");
@@ -130,7 +125,7 @@ __device__ __forceinline__ bool gather_slots(const unsigned long long* slots, ui
   }
   ok = __all_sync(0xffffffffu, ok);
 #pragma unroll
-  for (int v = 0; v < V; ++v) sum[v] = warp_sum_t(join(w[2 * v], w[2 * v + 1]));
+  for (int v = 0; v < V; ++v) sum[v] = warp_sum(join(w[2 * v], w[2 * v + 1]));
   return ok;
 }
 
@@ -252,8 +247,8 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pcg_team(Dev d, uint32_t fi
     if (own) put_word(z_mine + 6 * gi + a, __float_as_uint(z), epoch);
     double rz = 0.0, rr = 0.0;
     if (warp < nwarp) {
-      rz = warp_sum_t((double)r * (double)z);
-      rr = warp_sum_t((double)r * (double)r);
+      rz = warp_sum((double)r * (double)z);
+      rr = warp_sum((double)r * (double)r);
       if (lane == 0) {
         s_a[warp] = rz;
         s_b[warp] = rr;
@@ -339,24 +334,11 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pcg_team(Dev d, uint32_t fi
       }
       po = __fmaf_rn(beta, po, z);
       __syncthreads();
-      // Row sums of a part: the lanes' products by a reduce-scatter over
-      // bits 4 and 3, then a butterfly.
+      // Row sums of a part.
       auto reduce = [&](const float (&acc)[6], uint32_t node, uint32_t seg, bool store) {
+        float u, v;
+        row_sums(acc, lane, u, v);
         const bool b4 = (lane >> 4) & 1u, b3 = (lane >> 3) & 1u;
-        float h[3];
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          const float keep = b4 ? acc[q + 3] : acc[q], send = b4 ? acc[q] : acc[q + 3];
-          h[q] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-        }
-        const float g0 = __shfl_xor_sync(0xffffffffu, b3 ? h[0] : h[2], 8);
-        const float g1 = __shfl_xor_sync(0xffffffffu, h[1], 8);
-        float u = b3 ? h[2] + g0 : h[0] + g0, v = h[1] + g1;
-#pragma unroll
-        for (int off = 4; off > 0; off >>= 1) {
-          u += __shfl_xor_sync(0xffffffffu, u, off);
-          v += __shfl_xor_sync(0xffffffffu, v, off);
-        }
         float* out = part + (size_t)seg * 6 * nn + 6 * node + (b4 ? 3 : 0);
         if (store && (lane & 7u) == 0) out[b3 ? 2 : 0] = u;
         if (store && (lane & 15u) == 1) out[1] = v;
@@ -404,7 +386,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pcg_team(Dev d, uint32_t fi
       ++epoch;
       double pq_own = 0.0;
       if (warp < nwarp) {
-        pq_own = warp_sum_t((double)po * (double)qa);
+        pq_own = warp_sum((double)po * (double)qa);
         if (lane == 0) s_a[warp] = pq_own;
       }
       if (nwarp > 1) __syncthreads();
