@@ -25,8 +25,8 @@
 // up to 64 (12 columns, 72 registers of S per thread) and sixteen blocks of 8
 // warps up to 128 (24 columns, 144 registers).  Measured on B200 for one LM
 // iteration's solve, k_pcg against this kernel: 18 cameras and 29 PCG
-// iterations 300 -> 42 us, 48 cameras and 25 iterations 280 -> 60 us, a batch
-// of 48 windows of up to 36 cameras 554 -> 167 us over its three classes.
+// iterations 300 -> 43 us, 48 cameras and 25 iterations 280 -> 62 us, a batch
+// of 48 windows of up to 36 cameras 554 -> 173 us over its three classes.
 //
 // Every sum runs in an order fixed by the problem's own size, so a problem
 // solves the same alone and in any batch.  The cluster's blocks compute the

@@ -1,40 +1,48 @@
 // vlba_pcg_team.cu -- block-Jacobi PCG on reduced systems that fit the
-// shared memory of a team of SMs (past the cluster kernels' 128 cameras, up to
-// about 450 cameras of a dense system or 3,000 of a street).
+// registers and shared memory of a team of SMs (past the cluster kernels' 128
+// cameras, up to 576 cameras of a dense system, and 4,736, 2,808 or 1,328 of a
+// street whose tile rows reach 2, 6 or 12 rows to each side).
 //
 // The persistent k_pcg (vlba_kernels.cu) reads S again in every iteration,
 // sums partials of both triangles through global memory and crosses two grid
 // barriers: 20 us an iteration for 1,400 street cameras, whose S of 5 MB needs
 // none of that.  Here a problem has a team of blocks, one per SM; a block owns
 // consecutive cameras and keeps their rows of S (both triangles, the columns
-// of the tile rows they touch) in shared memory for the whole solve, so each
+// of the tile rows they touch) on the chip for the whole solve, so each
 // row of q = S p is summed where it is used and only z and three dots cross
 // blocks.  The same recurrence and stopping rule as k_pcg; two exchanges an
-// iteration:
+// iteration, three waits in a row:
 //
-//   q = S p for the block's rows, p.q           -> slot, all slots awaited
-//   x, r, z for the block's rows, r.z, r.r      -> z words and slot, awaited
+//   q = S p for the block's rows, p.q           -> slot; all slots awaited
+//   x, r, z for the block's rows, r.z, r.r      -> z words and slot; all slots
+//                                                  awaited, then the z words
 //   p = z + beta p for the columns the block reads
 //
 // An exchange has no barrier, flag or fence: every word published carries the
 // exchange's number beside its 32 bits of value (one 64-bit store, single-copy
-// atomic), so a reader that finds the number has the value.  A word is
-// written again only after its writer has seen every block's slot of the
-// exchange in between, which each block publishes after its own reads.  The
-// numbers go on from one solve to the next (team_epoch), so what an earlier
-// solve left is never taken for news (after a wait that gave up, whose blocks
-// may have stopped at different numbers, the host clears words and numbers).  A slot, and a block's z, has its 128-byte
-// lines to itself: with eight slots a line, polled by a hundred blocks while
-// eight write, an exchange took 3,800 cycles of 148 blocks, alone in a line
-// 1,800 (a counter barrier with loads behind it: 3,000).
+// atomic), so a reader that finds the number has the value.  A word is written
+// again only after its writer has seen every block's slot of the exchange in
+// between, which each block publishes after its own reads.  The numbers go on
+// from one solve to the next (team_epoch), so what an earlier solve left is never
+// taken for news (after a wait that gave up, whose blocks may have stopped at
+// different numbers, the host clears words and numbers).  A slot, and a block's
+// z, has its 128-byte lines to itself: with eight slots a line, polled by a
+// hundred blocks while eight write, an exchange took 3,800 cycles of 148 blocks,
+// alone in a line 1,800 (a counter barrier with loads behind it: 3,000; a kernel
+// of exchanges and nothing else on B200).
 //
-// What bounds an iteration is two trips through L2 (a store, then loads that
-// find it) and the chain of sums between them; the team is the smallest whose
-// blocks hold their rows in registers (polls lengthen with the team), else all
-// of the device with up to kExtra more parts a block.  A problem's team, its blocks'
-// rows and every sum's order follow from the problem alone; teams of several
-// problems run beside each other in rounds that fit the device, so a problem
-// solves the same alone and in any batch.  Every wait is bounded.
+// What bounds an iteration is the trips through L2 (a store, then loads that find
+// it) and the chain of sums between them; the team is the smallest whose blocks
+// hold their rows in registers (polls lengthen with the team), else all of the
+// device with up to kExtra more parts a block.  Measured on B200, k_pcg and this
+// kernel, us per PCG iteration of 60, the load of S in it: dense systems of 132
+// cameras 13.3 and 4.7, 300 10.2 and 5.3, 400 10.8 and 6.8, 500 11.2 and 7.9, 576
+// 12.0 and 8.8; streets of 300 cameras 14.2 and 4.7, 1,400 21.0 and 6.0, 2,800
+// 14.5 and 8.8: the line lies where the rows no longer fit.  A problem's team,
+// its blocks' rows and every sum's order follow from the problem alone; teams of
+// several problems run beside each other in rounds that fit the device, a launch
+// each, so a problem solves the same alone and in any batch.  Every wait is
+// bounded.
 
 #include <cuda_runtime.h>
 
