@@ -1353,7 +1353,7 @@ size_t Plan::device_bytes() const {
   b += tile_ij.size() * ((size_t)tb * tb * kBlock * 4 + 4 + 2 * (size_t)tb * 6 * 4);
   b += (size_t)num_var_cams * (4 + 4 + 4 + 4 + 36 * 4 + 6 * 4 * 6);
   b += tr_list.size() * 4 + (size_t)num_tile_rows * (4 + 4 + 16 * 8);
-  b += chunk_point_begin.size() * (4 + 8 + 8 + 8);
+  b += chunk_point_begin.size() * (4 + 8 + 8 + 8 + 8);
   // The team kernel's blocks, exchange words and tile lists (at most 16 blocks
   // where the cluster kernels solve unless the device places none of 16 blocks).
   for (size_t p = 0; p + 1 < prob_tr_begin.size(); ++p) {

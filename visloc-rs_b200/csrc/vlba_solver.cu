@@ -558,7 +558,7 @@ void upload_plan_once(Context* c, uint32_t max_records, const std::function<void
   // hold where that still gives each SM three blocks (five fit).  Measured on
   // B200 (update phase, a chunk a block and grouped): 24 windows of 200 to 5,000
   // points, 250 groups, 44 and 47 us; 32 windows 52 and 58; 48 windows, 490
-  // groups, 65 and 65; 60 windows 75 and 67; 512 windows 467 and 376.
+  // groups, 65 and 65; 60 windows 75 and 67; 512 windows 467 and 381.
   const std::vector<uint32_t> cost_group = cost_groups(P, 3u * (uint32_t)c->sm_count);
   d.num_cost_groups = (uint32_t)cost_group.size() / 2 - 1;
   // One copy for these and the teams' lists: a copy of its own costs each some
